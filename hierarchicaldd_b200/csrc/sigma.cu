@@ -425,9 +425,11 @@ void SigmaGpu::free_scratch(SigmaScratch& sc) {
     sc.bytes = 0;
 }
 
-void SigmaGpu::vcycle(cudaStream_t s, long long& launches, PhaseHook* hook) { vcycle(primary(), s, launches, hook); }
+void SigmaGpu::vcycle(bool u0_zero, cudaStream_t s, long long& launches, PhaseHook* hook) {
+    vcycle(primary(), u0_zero, s, launches, hook);
+}
 
-void SigmaGpu::vcycle(const SigmaScratch& sc, cudaStream_t s, long long& launches, PhaseHook* hook) {
+void SigmaGpu::vcycle(const SigmaScratch& sc, bool u0_zero, cudaStream_t s, long long& launches, PhaseHook* hook) {
     const int k = sc.nrhs;
     auto schur_apply = [&](int l, const float* u, float* out_tmp) {
         const SigmaLevel& L = lv[l];
@@ -436,23 +438,29 @@ void SigmaGpu::vcycle(const SigmaScratch& sc, cudaStream_t s, long long& launche
         L.aii.solve(S.aii, S.vb, S.vx, s, launches, hook, k, (long long)S.sn, (long long)S.sn);
         launch_csr(L.airT, S.vx, S.b, out_tmp, 1, s, launches, k, S.sn, S.si, S.si);  // tmp = b + Air^T vx
     };
-    auto smooth = [&](int l) {
+    // From u = 0 the step's subdomain solves are of zero vectors: tmp = b, so
+    // the interface solve reads b itself.  Every level starts there on the way
+    // down: one of its seven subdomain solves saved (whole solves: 128^3 127.1
+    // to 119.7 ms, 64^3 36.7 to 34.9 ms).
+    auto smooth = [&](int l, bool u_zero = false) {
         const SigmaScratch::Level& S = sc.lv[l];
-        schur_apply(l, S.u, S.tmp);
-        lv[l].arr_solve.solve(S.arr, S.tmp, S.u, s, launches, hook, k, (long long)S.si, (long long)S.si);
+        if (!u_zero) schur_apply(l, S.u, S.tmp);
+        lv[l].arr_solve.solve(S.arr, u_zero ? S.b : S.tmp, S.u, s, launches, hook, k, (long long)S.si,
+                              (long long)S.si);
     };
     for (int l = 0; l + 1 < M; ++l) {
         const SigmaLevel& L = lv[l];
         const SigmaScratch::Level& S = sc.lv[l];
         const SigmaScratch::Level& N = sc.lv[l + 1];
-        for (int i = 0; i < smoothing; ++i) smooth(l);
+        for (int i = 0; i < smoothing; ++i) smooth(l, i == 0 && (l > 0 || u0_zero));
         schur_apply(l, S.u, S.tmp);
         launch_csr(L.arr, S.u, S.tmp, S.r, 2, s, launches, k, S.si, S.si, S.si);  // r = tmp - Arr u
-        launch_fill(N.u, N.si * k, 0.0f, s, launches);
+        // Otherwise the next level's first solve writes all of its u.
+        if (smoothing == 0 && l + 2 < M) launch_fill(N.u, N.si * k, 0.0f, s, launches);
         launch_csr(L.prrT, S.r, nullptr, N.b, 0, s, launches, k, S.si, 0, N.si);  // b_{l+1} = Prr^T r
     }
     if (!bottom_exact) {
-        for (int i = 0; i < kBottomSmoothing; ++i) smooth(M - 1);
+        for (int i = 0; i < kBottomSmoothing; ++i) smooth(M - 1, i == 0 && (M > 1 || u0_zero));
     } else {
         const SigmaScratch::Level& B = sc.lv[M - 1];
         if (n_bottom > 0) {

@@ -312,13 +312,14 @@ struct SigmaGpu {
     // smoothing steps have not converged (HDD_COARSE_EXACT).
     void setup(const InterfaceHost& ih, int smoothing_iterations, cudaStream_t s, bool force_exact = false);
     void release();
-    // u[0] = sigma V-cycle(b[0]) (SIGMA_MULTIGRID_SOLVER.cpp:35-47), u[0] starting at 0,
-    // in the given scratch (default: the SigmaGpu's own).
-    void vcycle(cudaStream_t s, long long& launches, PhaseHook* hook = nullptr);
+    // u[0] = sigma V-cycle(b[0], u[0]) (SIGMA_MULTIGRID_SOLVER.cpp:35-47) in the
+    // given scratch (default: the SigmaGpu's own).  u0_zero: the caller has
+    // set u[0] = 0.
+    void vcycle(bool u0_zero, cudaStream_t s, long long& launches, PhaseHook* hook = nullptr);
     // With sc.nrhs = 2 or 4 it runs that many V-cycles at once (each
     // bit-identical to its V-cycle alone), every supernodal solve taking all
     // right-hand sides in one launch pair.
-    void vcycle(const SigmaScratch& sc, cudaStream_t s, long long& launches, PhaseHook* hook = nullptr);
+    void vcycle(const SigmaScratch& sc, bool u0_zero, cudaStream_t s, long long& launches, PhaseHook* hook = nullptr);
     SigmaScratch primary() const;
     void alloc_scratch(SigmaScratch& sc, cudaStream_t s, int nrhs = 1) const;
     // Most right-hand sides every plan of this hierarchy takes in one launch.

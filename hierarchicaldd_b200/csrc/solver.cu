@@ -562,7 +562,7 @@ void Solver::apply_preconditioner_launches(Work& w, const float* rr, float* zz) 
         NvtxRange sigma_range("Sigma_V_Cycle");
         Tm tm(this, w, 4);
         cuda_check(cudaMemsetAsync(w.sig.u0(), 0, sizeof(float) * w.sig.lv[0].si * w.k, w.stream), "memset u0");
-        for (int i = 0; i < opts.sigma_mg; ++i) sigma.vcycle(w.sig, w.stream, w.launches, &w == &w0 ? &hook : nullptr);
+        for (int i = 0; i < opts.sigma_mg; ++i) sigma.vcycle(w.sig, i == 0, w.stream, w.launches, &w == &w0 ? &hook : nullptr);
     }
     {
         Tm tm(this, w, 3);
@@ -631,7 +631,7 @@ void Solver::subdomain_dd(Work& w, const float* rr, float* zz, bool second) {
         NvtxRange sigma_range("Sigma_V_Cycle (second level)");
         Tm tm(this, w, 4);
         cuda_check(cudaMemsetAsync(w.sig2.u0(), 0, sizeof(float) * w.sig2.lv[0].si, w.stream), "memset u2");
-        for (int i = 0; i < opts.sigma_mg; ++i) sigma2.vcycle(w.sig2, w.stream, w.launches, &w == &w0 ? &hook : nullptr);
+        for (int i = 0; i < opts.sigma_mg; ++i) sigma2.vcycle(w.sig2, i == 0, w.stream, w.launches, &w == &w0 ? &hook : nullptr);
     }
     {
         // zz = 0, then the first- and second-level interface values.
@@ -665,7 +665,7 @@ void Solver::two_level_launches(Work& w, const float* rr, float* zz) {
         NvtxRange sigma_range("Sigma_V_Cycle");
         Tm tm(this, w, 4);
         cuda_check(cudaMemsetAsync(w.sig.u0(), 0, sizeof(float) * w.sig.lv[0].si, w.stream), "memset u1");
-        for (int i = 0; i < opts.sigma_mg; ++i) sigma.vcycle(w.sig, w.stream, w.launches, &w == &w0 ? &hook : nullptr);
+        for (int i = 0; i < opts.sigma_mg; ++i) sigma.vcycle(w.sig, i == 0, w.stream, w.launches, &w == &w0 ? &hook : nullptr);
     }
     {
         Tm tm(this, w, 3);
@@ -1150,7 +1150,7 @@ void Solver::sigma_vcycle_host(const float* b0, float* u0) {
     cuda_check(cudaMemcpyAsync(sigma.b0(), b0, n_if * sizeof(float), cudaMemcpyHostToDevice, stream), "H2D");
     cuda_check(cudaMemsetAsync(sigma.u0(), 0, n_if * sizeof(float), stream), "memset");
     sigma.clear_error(stream);
-    sigma.vcycle(stream, w0.launches);
+    sigma.vcycle(true, stream, w0.launches);
     cuda_check(cudaMemcpyAsync(u0, sigma.u0(), n_if * sizeof(float), cudaMemcpyDeviceToHost, stream), "D2H");
     sync();
     check_waits();
