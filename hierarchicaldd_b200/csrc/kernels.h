@@ -67,9 +67,10 @@ struct TileGeom;
 
 // Whole-grid V-cycle (kernels_vcycle_global.cu), for domains whose coarse
 // levels couple subdomain boxes: level l is a dense x-slowest grid of
-// dims[l] cells with compact8 flags f[l]; u, b, r are its vectors (level 0
-// staged from and back to the tiled vectors).  Coarse r must be zero where a
-// level is not Active (allocated zeroed; never written there).
+// dims[l] cells with compact8 flags f[l]; u, b, r are its vectors, t a second
+// copy of u (level 0 staged from and back to the tiled vectors).  Coarse r
+// must be zero where a level is not Active (allocated zeroed; never written
+// there).
 struct GlobalVcycleArgs {
     int levels;
     int dims[kMaxLevels][3];
@@ -77,6 +78,7 @@ struct GlobalVcycleArgs {
     float* u[kMaxLevels];
     float* b[kMaxLevels];
     float* r[kMaxLevels];
+    float* t[kMaxLevels];
     int n_vcycles, interior_itr, boundary_itr, bottom_itr;
     int halo_from_u, zero_init;   // as in VcycleArgs
     VcycleWeights w;

@@ -343,7 +343,7 @@ void Solver::alloc_vectors(Work& w) {
     for (int l = 0; l < kMaxLevels; ++l) {
         const bool on = L.global_vcycle && l < L.opt.vlevels;
         const size_t c = on ? (size_t)L.g_dims[l][0] * L.g_dims[l][1] * L.g_dims[l][2] : 0;
-        for (DevBuf<float>* v : {&w.gu[l], &w.gb[l], &w.gr[l]}) {
+        for (DevBuf<float>* v : {&w.gu[l], &w.gb[l], &w.gr[l], &w.gt[l]}) {
             if (on) { v->alloc(c); v->zero(w.stream); }
             else v->release();
         }
@@ -394,7 +394,7 @@ size_t Solver::work_bytes(int k) const {
     if (opts.precision_mode == HDD_PRECISION_MIXED) t += std::max<size_t>(N, 1) * 8 * k;
     t += (P * 12 + 128 + sizeof(PcgScalars) + 12) * k;
     if (L.global_vcycle)
-        for (int l = 0; l < L.opt.vlevels; ++l) t += 12 * (size_t)L.g_dims[l][0] * L.g_dims[l][1] * L.g_dims[l][2];
+        for (int l = 0; l < L.opt.vlevels; ++l) t += 16 * (size_t)L.g_dims[l][0] * L.g_dims[l][1] * L.g_dims[l][2];
     return t + sigma.scratch_bytes(k) + (sigma2.lv.empty() ? 0 : sigma2.scratch_bytes(k));
 }
 
@@ -468,6 +468,7 @@ void Solver::run_vcycle(Work& w, float* u, const float* bb, int halo_from_u, int
             ga.u[l] = w.gu[l].p;
             ga.b[l] = w.gb[l].p;
             ga.r[l] = w.gr[l].p;
+            ga.t[l] = w.gt[l].p;
         }
         ga.n_vcycles = nv;
         ga.interior_itr = a.interior_itr;

@@ -84,7 +84,7 @@ struct Work {
     DevBuf<int> active, first, replace;
     DevBuf<float> x, b, r, z, s, q;
     DevBuf<float> hr;       // two-level DD: the V-cycle's lower-face residual input
-    DevBuf<float> gu[kMaxLevels], gb[kMaxLevels], gr[kMaxLevels];  // whole-grid V-cycle levels
+    DevBuf<float> gu[kMaxLevels], gb[kMaxLevels], gr[kMaxLevels], gt[kMaxLevels];  // whole-grid V-cycle levels
     DevBuf<double> xd;      // precision form: the FP64 iterate (x is its FP32 rounding)
     DevBuf<float> dense;    // staging buffer in the caller's dense layout
     DevBuf<double> partial, sums;
@@ -118,7 +118,7 @@ struct Work {
         size_t t = 0;
         for (const DevBuf<float>* v : {&x, &b, &r, &z, &s, &q, &hr, &dense, &partial_max, &scalars_f})
             t += v->n * sizeof(float);
-        for (int l = 0; l < kMaxLevels; ++l) t += (gu[l].n + gb[l].n + gr[l].n) * sizeof(float);
+        for (int l = 0; l < kMaxLevels; ++l) t += (gu[l].n + gb[l].n + gr[l].n + gt[l].n) * sizeof(float);
         t += (partial.n + sums.n + xd.n) * sizeof(double) + scal.n * sizeof(PcgScalars);
         t += (active.n + first.n + replace.n) * sizeof(int);
         return t + (own_sig ? sig.bytes : 0) + (own_sig2 ? sig2.bytes : 0);
