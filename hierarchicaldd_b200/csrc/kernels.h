@@ -43,7 +43,6 @@ struct VcycleArgs {
     int n_vcycles, interior_itr, boundary_itr, bottom_itr;
     int halo_from_u;           // 1: halo planes hold interface values read from u
     int zero_init;             // 1: interior u starts at zero
-    int cluster;               // CTAs per subdomain for sub 16 (1 or 2); sub 32 always uses 4
     float inv_diag[8];         // omega / face_count (float division on the host)
     float restrict_w[64];      // (1/8,3/8,3/8,1/8)^3 tensor weights
     float prolong_w[8];        // 4 * (3/4,1/4)^3 tensor weights

@@ -429,11 +429,9 @@ VcycleArgs Solver::vcycle_args(float* u, const float* bb, int halo_from_u, int z
     a.bottom_itr = 200;  // CPU/SPGrid_Library/SPGrid_V_Cycle_Helper.h:179
     a.halo_from_u = halo_from_u;
     a.zero_init = zero_init;
-    a.cluster = 1;
     a.nslots = 1;
     a.slot_stride = 0;
     a.active = nullptr;
-    if (const char* e = std::getenv("HDD_VCYCLE_CLUSTER")) a.cluster = std::atoi(e);
     // Correction weights omega/face_count with omega = (float)(2/3)
     // (SPGrid_Correction_Legacy.h:35,76), divided in float on the host.
     const float omega = (float)(2. / 3.);
