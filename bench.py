@@ -153,7 +153,7 @@ def set_domain(s, d):
 
 
 PHASES = ["vcycle", "laplace", "pcg_vector", "interface", "sigma_vcycle", "dense_tile_copy",
-          "sn_forward", "sn_backward"]
+          "sn_solve", "unused"]
 
 
 def one_solve(args):
@@ -745,9 +745,9 @@ def main():
     # device time is the headline.
     hbm, peak_kind = peaks()
     vbox = d.sub_size[0] // 2 if m.get("multilevel") else d.sub_size[0]  # V-cycle box and tile edge
-    kernels = {0: "vcycle_cluster_kernel" if vbox == 32 else "vcycle_kernel",
+    kernels = {0: "vcycle_kernel_32" if vbox == 32 else "vcycle_kernel",
                1: "laplace_dot_march_kernel" if vbox in (8, 16, 32) else "laplace_dot_kernel",
-               6: "sn_forward_kernel", 7: "sn_backward_kernel"}
+               6: "sn_solve"}
     per_kernel = {}
     for i, kname in kernels.items():
         if cnt[i] == 0 or ms[i] <= 0:

@@ -30,6 +30,7 @@ SOURCES = [
     "sigma.cu",
     "sn_plan.cpp",
     "sn_solve.cu",
+    "sn_resident.cu",
     "solver.cu",
     "noalloc.cu",
     "velocity.cu",

@@ -150,11 +150,10 @@ void build_layout(const Options& opt, const uint32_t* flags, DomainLayout& L) {
     for (int a = 0; a < 3; ++a) {
         if (opt.size[a] < 3) throw Error(HDD_ERR_INVALID_ARGUMENT, "size must be >= 3 on every axis");
         int s = opt.sub[a];
-        // The resident V-cycle keeps a subdomain's levels on chip: one CTA for
-        // 8^3 and 16^3 boxes, a 4-CTA cluster for 32^3.  A 64^3 box (the
-        // reference Test_Bench default, CPU/Test_Bench_3D/main.cpp:247) needs
-        // 64^3 x 8 B of level-0 state, more than a 16-CTA cluster's shared
-        // memory, and 4^3 boxes have no coarse level worth a launch; both are
+        // The resident V-cycle keeps a subdomain's levels on chip: one CTA
+        // per box up to 32^3.  A 64^3 box (the reference Test_Bench default,
+        // CPU/Test_Bench_3D/main.cpp:247) needs 64^3 x 8 B of level-0 state,
+        // more than the shared memory of 16 CTAs, and 4^3 boxes have no coarse level worth a launch; both are
         // refused here, before any setup work.
         if (s != 8 && s != 16 && s != 32)
             throw Error(HDD_ERR_UNSUPPORTED, "sub_size must be 8, 16 or 32 (got " + std::to_string(s) + ")");

@@ -196,13 +196,14 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
         L.vx = dev::alloc_zero<float>(std::max(L.n_int, 1), bytes, s);
         device_bytes += bytes;
 
-        // Factorisations.
+        // Factorisations, one per distinct subdomain matrix.
+        const std::vector<int> rep = interior_classes(ih, l);
         std::vector<SnFactor> aii(ih.n_sub);
         std::vector<std::string> err(ih.n_sub);
 #pragma omp parallel for schedule(dynamic)
         for (int sd = 0; sd < ih.n_sub; ++sd) {
             try {
-                if (ih.Aii[l][sd].rows == 0) continue;
+                if (ih.Aii[l][sd].rows == 0 || rep[sd] != sd) continue;
                 aii[sd].analyze(ih.Aii[l][sd], interior_positions(ih, l, sd));
                 aii[sd].factor(ih.Aii[l][sd], eps);
                 if (l + 1 < M) aii[sd].build_solve_blocks();
@@ -221,7 +222,7 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
             std::vector<const SnFactor*> fs;
             std::vector<int> offs;
             for (int sd = 0; sd < ih.n_sub; ++sd)
-                if (aii[sd].n > 0) { fs.push_back(&aii[sd]); offs.push_back(off[sd]); }
+                if (ih.Aii[l][sd].rows > 0) { fs.push_back(&aii[rep[sd]]); offs.push_back(off[sd]); }
             L.aii.build(fs, offs, s, d_err);
             L.arr_solve.build({&arrf}, {0}, s, d_err);
             device_bytes += L.aii.bytes + L.arr_solve.bytes;
@@ -247,7 +248,7 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
                         tv.assign(Air.rows, 0.0);
                         for (int r = 0; r < Air.rows; ++r)
                             for (int p = Air.ptr[r]; p < Air.ptr[r + 1]; ++p) tv[r] += Air.val[p] * xv[Air.col[p]];
-                        aii[sd].solve(tv.data());
+                        aii[rep[sd]].solve(tv.data());
                         for (int r = 0; r < Air.rows; ++r)
                             for (int p = Air.ptr[r]; p < Air.ptr[r + 1]; ++p) yv[Air.col[p]] += Air.val[p] * tv[r];
                     }
@@ -280,7 +281,7 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
                 std::vector<const SnFactor*> fs;
                 std::vector<int> offs;
                 for (int sd = 0; sd < ih.n_sub; ++sd)
-                    if (aii[sd].n > 0) { fs.push_back(&aii[sd]); offs.push_back(off[sd]); }
+                    if (ih.Aii[l][sd].rows > 0) { fs.push_back(&aii[rep[sd]]); offs.push_back(off[sd]); }
                 L.aii.build(fs, offs, s, d_err);
                 L.arr_solve.build({&arrf}, {0}, s, d_err);
                 device_bytes += L.aii.bytes + L.arr_solve.bytes;

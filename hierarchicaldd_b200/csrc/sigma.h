@@ -109,9 +109,8 @@ protected:
     ~PhaseHook() = default;
 };
 
-// Timing phases of the supernodal solve kernels.
-constexpr int kPhaseSnForward = 6;
-constexpr int kPhaseSnBackward = 7;
+// Timing phase of the supernodal solves (both directions).
+constexpr int kPhaseSolve = 6;
 
 // Host reference of a solve plan (sn_plan.cpp): the fronts of a batch of
 // independent factorisations with concatenated unknowns and the FP32
@@ -136,22 +135,34 @@ struct PlanHost {
 const std::vector<std::array<int, 3>>* interface_positions(const InterfaceHost& ih, int l);
 const std::vector<std::array<int, 3>>* interior_positions(const InterfaceHost& ih, int l, int sd);
 
+// Subdomains of level l with equal interior systems (matrix and, where known,
+// DOF positions relative to the first DOF): entry sd is the first subdomain
+// whose system equals sd's.  Equal systems have equal factors.
+std::vector<int> interior_classes(const InterfaceHost& ih, int l);
+
 // Factorisations of one interface solve as the sigma solver builds them
 // (A + 1e-5 I, ordering from the positions, explicit solve blocks) and the
 // plan over them: kind 0 = Arr of level l, kind 1 = Aii of every subdomain of
 // level l with the unknowns concatenated in subdomain order.
 void interface_solve_plan(const InterfaceHost& ih, int kind, int l, std::vector<SnFactor>& factors, PlanHost& plan);
 
-// One unit of device work of a supernodal solve, taken by a CTA of the
-// persistent solve kernels (sn_solve.cu).  With front >= 0, forward: rows
-// [r0, r0+rows) of front `front` times its columns [c0, c0+ncols); when a row
-// block is split into nk > 1 column blocks, the partial sums go to `part` and
-// the last task of the block (counter `chunk`) adds them in order; backward:
-// columns [r0, r0+rows) of the front.  With front < 0, a bundle of `rows`
-// small fronts (listed from index r0 of the plan's bundle list), one per warp.
-struct SnTask {
+// One unit of device work of the fronts above a plan's cut trees, taken by a CTA
+// of the persistent task kernel (sn_solve.cu), with what the CTA needs of the
+// front.  Forward: rows [r0, r0+rows) of front `front` times its columns [c0,
+// c0+ncols); backward: columns [r0, r0+rows) over rows [c0, c0+ncols).  A block
+// split into nk > 1 tasks writes partial sums to `part`, which the last task to
+// finish (counter `chunk`) adds in order.
+struct alignas(16) SnTask {
     int front, r0, rows, c0, ncols, k, nk, chunk;
-    long long part;
+    int nj, m, col0, parent;       // the front's columns, rows, first unknown, parent (-1: root)
+    int upd, child_b, child_e;     // its update vector; the children it waits for
+    int kids, cw, pad;             // whether it has children at all; backward: columns per warp
+    long long part, fw, rows_off, gp, ge;  // offsets of partial sums, coefficients, rows, gather lists
+};
+
+// What a ResidentPlan's launches write besides the solution.
+struct ResidentScratch {
+    double *upd = nullptr, *y = nullptr;
 };
 
 // The device buffers one supernodal solve writes (split-block partial sums,
@@ -161,6 +172,7 @@ struct SnTask {
 struct PlanScratch {
     double *part = nullptr, *upd = nullptr, *ynew = nullptr, *xnew = nullptr;
     int* ctr = nullptr;
+    ResidentScratch res;
     int* err = nullptr;
     bool own_err = false;
     // The persistent launches use 1/grid_div of the plan's CTAs (rounded up),
@@ -170,46 +182,102 @@ struct PlanScratch {
     int nrhs = 1;  // right-hand sides the buffers hold (1, 2 or 4)
 };
 
+struct RGroup;
+struct RWarp;
+
+// Cut trees: the update vectors (written going up) and the solution (read
+// coming down) of the plan above them; right-hand side j at + j ld.
+struct TopVectors {
+    double* upd = nullptr;
+    const double* x = nullptr;
+    long long ld_upd = 0, ld_x = 0;
+    int* ctr = nullptr;       // counters that the forward launch clears
+    long long n_ctr = 0;
+};
+
+// Plan of solves with one CTA per elimination tree, or per group of them
+// (sn_resident.cu).
+struct ResidentPlan {
+    static constexpr size_t kMaxSmem = 226 * 1024;
+    // Trees of one factor solved by one CTA: fronts first .. last (the root) of
+    // each; top: where the root's update vector goes in the plan above (-1: the
+    // root has none).  ext_off: index of the factor's unknown 0 in the solution
+    // of the plan above.
+    struct Tree { int first, last, top; };
+    struct Shape {
+        const SnFactor* F = nullptr;
+        std::vector<Tree> trees;
+        int ext_off = 0;
+    };
+    bool cut = false;                   // cut trees: separate forward and backward launches
+    int n = 0, max_n = 0, ngroups = 0;  // unknowns; largest vector; CTAs of one solve (0: no plan)
+    int km = 1, nt = 256;               // trees per CTA (1, 2 or 4), threads per CTA
+    int entries = 0;                    // doubles of a CTA's trees in shared memory
+    int resident = 1;                   // CTAs that fit on the device
+    size_t smem = 0, bytes = 0;         // shared memory per CTA; device bytes
+    long long upd_len = 0, y_len = 0;   // doubles of a ResidentScratch's buffers
+    double solve_bytes = 0;             // algorithmic bytes of one solve, both directions
+    bool global_slots = false;          // update entries in global memory (they do not fit shared memory)
+    RGroup* d_groups = nullptr;
+    RWarp* d_warps = nullptr;
+    int *d_off = nullptr, *d_perm = nullptr, *d_ext = nullptr;
+    char* d_stream = nullptr;           // every class's warp streams: coefficients and indices
+    int* d_gate = nullptr;
+    // Shared memory of the rings and of k trees of `entries` doubles each.
+    static size_t smem_bytes(int entries, int k, int nt);
+    // Whole factors: factors[i] solves the unknowns from offsets[i] on; members
+    // given the same SnFactor form a class that shares its coefficients.  False
+    // when a CTA's shared memory does not hold the trees.
+    bool build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s);
+    // Cut trees: shape i of the factor whose unknowns start at offsets[i].
+    bool build_cut(const std::vector<Shape>& shapes, const std::vector<int>& offsets, cudaStream_t s);
+    void release();
+    // mode: 0 whole trees, both directions; 1 / 2 the forward / backward half of cut trees.
+    void launch(int mode, const ResidentScratch& sc, const TopVectors& top, int* err, int grid_div,
+                long long spin_limit, const float* b_old, float* x_old, cudaStream_t s, int nrhs, long long ld_b,
+                long long ld_x) const;
+    // Test seam: while nonzero, every solve of whole trees waits for it (bounded) and raises the error word.
+    void set_gate(int v, cudaStream_t s);
+
+private:
+    bool build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<int>>& members, cudaStream_t s);
+};
+
 // Device plan for a batch of independent supernodal triangular solves.
 struct SolvePlan {
+    // One CTA per tree: the whole plan, or (cut) the lower trees of a task plan
+    // that has the fronts above them.
+    ResidentPlan res;
+    bool whole_resident() const { return res.ngroups > 0 && !res.cut; }
     int n = 0;                       // total unknowns (concatenated)
-    int nsn = 0;
-    int max_front = 0;
-    int n_fwd = 0, n_bwd = 0;        // task counts
-    int n_ctr = 0;                   // ints in the counter block
-    int grid = 0;                    // persistent CTAs per launch (one right-hand side)
-    int grids[3] = {0, 0, 0};        // ... for 1, 2 and 4 right-hand sides (0: shared memory too small)
-    int kmax = 1;                    // most right-hand sides one launch takes
-    int nt = 256;                    // threads per CTA (128 for plans of many factors)
-    int ntasks_f = 0, ntasks_b = 0;  // tasks, forward / backward
-    double fwd_bytes = 0, bwd_bytes = 0;  // algorithmic bytes of one forward / backward launch
-    int *d_col0 = nullptr, *d_ncol = nullptr, *d_nrow = nullptr, *d_parent = nullptr;
-    int *d_rows = nullptr; long long *d_rows_off = nullptr;
-    int *d_child_ptr = nullptr, *d_child = nullptr;
-    long long* d_relmap_off = nullptr; int* d_relmap = nullptr;
-    long long *d_gp_off = nullptr, *d_ge_off = nullptr;  // per front: gather-list offsets
-    int *d_gptr = nullptr, *d_gent = nullptr;           // gather lists (see sn_solve.cu)
-    long long* d_upd_off = nullptr;
-    long long* d_fw_off = nullptr;   // per front: float offset of Fw (leading dimension round4(m))
-    int *d_ntf = nullptr, *d_ntb = nullptr;  // tasks per front, forward / backward
+    int nsn = 0, ntop = 0;           // fronts; those above the cut trees
+    int max_front = 0;               // of those
+    int n_fwd = 0, n_tasks = 0;      // forward tasks, all tasks
+    int ld_ctr = 0;                  // ints of one right-hand side's counters
+    int grid = 0;                    // persistent CTAs of the task launch
+    int kmax = 1;                    // most right-hand sides one solve takes
+    double solve_bytes = 0;          // algorithmic bytes of one solve, both directions
+    int *d_rows = nullptr, *d_child = nullptr;
+    int *d_gptr = nullptr, *d_gent = nullptr;  // gather lists (see sn_solve.cu)
+    int *d_ntf = nullptr, *d_ntb = nullptr;    // tasks per front, forward / backward
     int* d_perm = nullptr;           // new -> old (concatenated)
-    SnTask *d_fwd = nullptr, *d_bwd = nullptr;
-    int *d_bfwd = nullptr, *d_bbwd = nullptr;  // fronts of the forward / backward bundles
-    float* d_fw = nullptr;           // Fw blocks of all fronts
-    double* d_part = nullptr;        // partial sums of split row blocks
+    SnTask* d_tasks = nullptr;
+    float* d_fw = nullptr;           // Fw blocks of the fronts above
+    ResidentScratch d_res;
+    double* d_part = nullptr;        // partial sums of split blocks
     double* d_upd = nullptr;         // update vectors
     double* d_ynew = nullptr;        // forward result in new order
     double* d_xnew = nullptr;        // backward result in new order
-    int* d_ctr = nullptr;            // tickets, completion and chunk counters
+    int* d_ctr = nullptr;            // ticket, completion and chunk counters
     int* d_err = nullptr;            // set when a bounded wait gives up
     bool own_err = false;            // d_err allocated by this plan (else shared)
     long long spin_limit = 1LL << 22;  // polls of a bounded wait before it gives up
     int stall_front = -1, stall_ntf = 0;  // front used by stall_dependency and its task count
     size_t bytes = 0;
     // shared_err: an error word shared with other plans (owned by the caller),
-    // or null for a word of the plan's own.
+    // or null for a word of the plan's own.  shrink: divides the size of cut trees.
     void build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s,
-               int* shared_err = nullptr);
+               int* shared_err = nullptr, double shrink = 1);
     void release();
     long long part_len = 0, upd_len = 0;  // doubles in a scratch's partial-sum and update buffers
     // x_old = (A+eps I)^{-1} b_old (both in the concatenated original order),
@@ -217,8 +285,8 @@ struct SolvePlan {
     void solve(const float* b_old, float* x_old, cudaStream_t s, long long& launches,
                PhaseHook* hook = nullptr) const;
     // With nrhs = 2 or 4 it solves that many systems at once: right-hand side
-    // j at b_old + j ld_b, solution at x_old + j ld_x, each coefficient read
-    // once for all of them; each solution is bit-identical to its solve alone.
+    // j at b_old + j ld_b, solution at x_old + j ld_x, one system's work beside
+    // the other's; each solution is bit-identical to its solve alone.
     void solve(const PlanScratch& sc, const float* b_old, float* x_old, cudaStream_t s, long long& launches,
                PhaseHook* hook = nullptr, int nrhs = 1, long long ld_b = 0, long long ld_x = 0) const;
     // Scratch for another solve context (error word shared_err, or its own),
@@ -227,15 +295,7 @@ struct SolvePlan {
     static void free_scratch(PlanScratch& sc);
     PlanScratch primary() const;
     // Device bytes alloc_scratch takes (without a shared error word).
-    size_t scratch_bytes() const {
-        if (nsn == 0) return 0;
-        return 8 * (size_t)(part_len + upd_len) + 16 * (size_t)std::max(n, 1) + 4 * (size_t)std::max(n_ctr, 1) + 4;
-    }
-    size_t scratch_bytes(int nrhs) const {
-        if (nsn == 0) return 0;
-        return nrhs * (8 * (size_t)(part_len + upd_len) + 16 * (size_t)std::max(n, 1)) +
-               4 * (size_t)std::max(n_ctr, 1) + 4;
-    }
+    size_t scratch_bytes(int nrhs = 1) const;
     int error_flag(cudaStream_t s) const;
     // Test seam: on = raise the forward task count that one front's parent
     // waits for by one, so that wait can never be satisfied and runs into its
@@ -318,7 +378,7 @@ struct SigmaGpu {
     void vcycle(bool u0_zero, cudaStream_t s, long long& launches, PhaseHook* hook = nullptr);
     // With sc.nrhs = 2 or 4 it runs that many V-cycles at once (each
     // bit-identical to its V-cycle alone), every supernodal solve taking all
-    // right-hand sides in one launch pair.
+    // right-hand sides in the same launches.
     void vcycle(const SigmaScratch& sc, bool u0_zero, cudaStream_t s, long long& launches, PhaseHook* hook = nullptr);
     SigmaScratch primary() const;
     void alloc_scratch(SigmaScratch& sc, cudaStream_t s, int nrhs = 1) const;

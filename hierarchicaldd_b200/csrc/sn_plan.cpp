@@ -8,7 +8,10 @@
 // check the device solve against it.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
+#include <cstring>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "sigma.h"
@@ -96,6 +99,51 @@ const std::vector<std::array<int, 3>>* interior_positions(const InterfaceHost& i
     if (l >= (int)ih.aii_xyz.size() || sd >= (int)ih.aii_xyz[l].size()) return nullptr;
     if ((int)ih.aii_xyz[l][sd].size() != ih.Aii[l][sd].rows) return nullptr;
     return &ih.aii_xyz[l][sd];
+}
+
+std::vector<int> interior_classes(const InterfaceHost& ih, int l) {
+    const int n = ih.n_sub;
+    std::vector<uint64_t> key(n);
+    auto positions = [&](int sd) { return interior_positions(ih, l, sd); };
+#pragma omp parallel for schedule(dynamic)
+    for (int sd = 0; sd < n; ++sd) {
+        uint64_t h = 1469598103934665603ull;
+        auto mix = [&](uint32_t v) { h = (h ^ v) * 1099511628211ull; };
+        const CsrF& A = ih.Aii[l][sd];
+        mix((uint32_t)A.rows);
+        for (int p : A.ptr) mix((uint32_t)p);
+        for (int c : A.col) mix((uint32_t)c);
+        for (float v : A.val) {
+            uint32_t u;
+            std::memcpy(&u, &v, 4);
+            mix(u);
+        }
+        key[sd] = h;
+    }
+    auto same = [&](int a, int b) {
+        const CsrF &A = ih.Aii[l][a], &B = ih.Aii[l][b];
+        if (A.rows != B.rows || A.cols != B.cols || A.ptr != B.ptr || A.col != B.col) return false;
+        if (A.val.size() != B.val.size()) return false;
+        if (!A.val.empty() && std::memcmp(A.val.data(), B.val.data(), A.val.size() * sizeof(float)) != 0) return false;
+        const auto *pa = positions(a), *pb = positions(b);
+        if (!pa || !pb) return !pa && !pb;
+        for (size_t i = 0; i < pa->size(); ++i)
+            for (int x = 0; x < 3; ++x)
+                if ((*pa)[i][x] - (*pa)[0][x] != (*pb)[i][x] - (*pb)[0][x]) return false;
+        return true;
+    };
+    // Equal keys first to last; a key shared by different systems keeps them apart.
+    std::vector<int> rep(n);
+    std::unordered_map<uint64_t, std::vector<int>> reps;
+    for (int sd = 0; sd < n; ++sd) {
+        rep[sd] = sd;
+        std::vector<int>& r = reps[key[sd]];
+        bool found = false;
+        for (int c : r)
+            if (same(c, sd)) { rep[sd] = c; found = true; break; }
+        if (!found) r.push_back(sd);
+    }
+    return rep;
 }
 
 void interface_solve_plan(const InterfaceHost& ih, int kind, int l, std::vector<SnFactor>& factors, PlanHost& plan) {

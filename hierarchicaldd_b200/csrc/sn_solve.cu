@@ -14,24 +14,34 @@
 // to FP32 once, at its output, like the FP64 substitution it replaces up to
 // the rounding of the stored coefficients.
 //
-// Each direction is ONE persistent launch.  Its work is a list of tasks in
-// topological order (forward: children before parents; backward: parents
-// before children); CTAs take tasks by ticket and, before starting one, wait
-// on per-front completion counters of the fronts it depends on.  A task only
-// ever waits on tasks with smaller tickets, which running CTAs already hold,
-// so the walk always progresses; every wait is bounded anyway and raises the
-// plan's error word when it gives up.  Data produced by other CTAs in the same
-// launch is read with L2-coherent loads after an acquire of the counter.
+// A plan whose trees each fit one CTA is solved by sn_resident.cu alone.
+// Otherwise the lower trees of every factor (most of the fronts, little of
+// the work each) go there, forward before and backward after the launch of
+// this file, which has the fronts above them.
 //
-// Small fronts (a few row chunks times few columns) go in bundles of one per
-// warp, so that many short dependency chains run per CTA.  Other
-// forward tasks are row blocks of up to kRB rows; a CTA splits its threads
-// into row lanes x column slices and adds the slices in a fixed order.  Tall
-// fronts whose row block needs more than kCC columns are split into column
-// blocks: each writes its partial sums and the last one to finish adds them in
-// column order, so every result is independent of scheduling.  Backward tasks
-// are blocks of kBC columns, one warp per column group, lanes striding down
-// the contiguous columns.
+// That launch is persistent and does both directions.  Its work is a list of
+// tasks in topological order (forward: children before parents; then
+// backward: parents before children); CTAs take them by ticket and, before
+// starting one, wait on per-front completion counters of the fronts it depends
+// on.  A task only ever waits on tasks with smaller tickets.  A CTA takes its
+// next ticket while it works on the current one; the smallest unfinished
+// ticket is then still the current one of a running CTA, so the walk always
+// progresses.  Every wait is bounded anyway and raises the plan's error word
+// when it gives up.  Data produced by other CTAs in the same launch is read
+// with L2-coherent loads after an acquire of the counter.
+//
+// Forward tasks are row blocks of up to kRB rows times up to kCC columns (taller
+// triangles: several column blocks, whose partial sums the last one to finish
+// adds in column order); backward tasks are column blocks, one warp per column
+// group, lanes striding down the contiguous columns, tall ones cut into row
+// chunks the same way.  So every result is independent of scheduling.
+//
+// What bounds it: near the top of a tree a few fronts a level follow one
+// another, so the time from one front's end to the next one's.  Everything a
+// task needs that does not depend on the fronts below (its record, its
+// coefficients, the gather indices of its inputs) is loaded before it waits;
+// after the wait come one load of the inputs, the products, one reduction and
+// the release of its counter.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,7 +49,8 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
-#include <mutex>
+#include <map>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -49,58 +60,65 @@
 namespace hdd {
 namespace {
 
-// Threads per CTA: a plan of many independent factors (the subdomain
-// interiors) runs 64-thread CTAs, many of them per SM for its many short
-// tasks; a plan of one factor (the interface) runs 256-thread CTAs, which do
-// its tall fronts in fewer tasks.  Measured at 256^3, level-0 interior plan
-// forward / backward: 801 / 836 us with 256 threads, 650 / 760 with 128,
-// 577 / 711 with 64; level-0 interface plan: 480 / 596 us with 256 threads,
-// 662 / 731 with 128, 703 / 565 with 512.
-constexpr int kNTInterior = 64, kNTInterface = 256;
-constexpr int kRB = 128;                 // rows per forward row block
-constexpr int kCC = 128;                 // columns per forward column block
-// Small fronts per bundle (one per warp) and columns per backward task (4 per
-// warp), for NT threads.
-__host__ __device__ constexpr int warps_of(int nt) { return nt / 32; }
-__host__ __device__ constexpr int bc_of(int nt) { return 4 * (nt / 32); }
-// CTAs per SM the register budget is sized for (K right-hand sides, NT threads).
-__host__ __device__ constexpr int min_blocks(int k, int nt) { return (k == 1 ? 1280 : (k == 2 ? 768 : 512)) / nt; }
-constexpr int kSmallM = 256;             // rows of a front solved by one warp
-constexpr int kSmallLoads = 128;         // ... when its row chunks x columns stay below this
-
-constexpr int kBundleLevel = 2048;       // bundle only on levels with at least this many small fronts
-
-bool small_front(int m, int nj) { return m <= kSmallM && ((m + 31) / 32) * nj <= kSmallLoads; }
+constexpr int kNT = 256;      // threads per CTA
+constexpr int kPerSM = 2;     // CTAs per SM the register budget is sized for
+constexpr int kRB = 128;      // rows per forward task
+constexpr int kCC = 128;      // columns per forward task of a split block
+constexpr int kWhole = 256;   // ... and the most columns of an unsplit one
+constexpr int kBLoads = 16;   // coefficient quads a lane loads in a backward task
+// Backward tasks: 8 warps x kCW columns by kBLoads / kCW row quads per lane:
+// 32 columns x 512 rows, or 16 x 1024 for taller fronts, so that a front of up
+// to 1024 rows needs no partial sums.
+constexpr int kWarps = kNT / 32;
+constexpr int kTallRows = 512;
+__host__ __device__ constexpr int cols_of(int cw) { return kWarps * cw; }
+__host__ __device__ constexpr int rows_of(int cw) { return kBLoads / cw * 128; }
+// Partial sums a tree may need beside its unknowns.
+constexpr int kPartMax = 4096;
+// The trees one CTA takes of a cut plan: at most a cut of front_weight() and a
+// vector of kCutLen.  A front costs its coefficients and about what 1000
+// coefficients do for its operations (the trees of sparse domains are thousands
+// of tiny fronts).  The cut grows with the plan so that its trees are about one
+// CTA per SM: larger ones would take longer than the task levels they save,
+// smaller ones leave more of those.  Measured (us per
+// solve at cuts of total/280 and at least 16000, total/250 and 36000,
+// total/170 and 48000): interface of 40x36x44, sub 8 (9 MB) 82, 81, 75; 64^3,
+// sub 16 (15 MB) 86, 87, 84; second level of 192^3, sub 32 (39 MB) 94, 90, 101;
+// 128^3 (63 MB) 121, 124, 119; sparse 128^3 43, 41, 31.
+constexpr double kCutMin = 48000, kCutMax = 200000, kCutShare = 220;
+// One CTA per whole tree takes as long as its largest tree's weight; cut, about
+// as long as kCutCost, and a kCutRate-th of all.  Measured (us
+// per solve): 8 interiors of 32^3 whole 158, cut 69; 16, 32 and 48 of them cut
+// 81, 104 and 153; 64 whole 165; a 16^3 domain's interface (564 unknowns) whole
+// 27, cut 43.
+constexpr double kCutCost = 300000, kCutRate = 80;
+constexpr int kCutLen = 8192;
 
 struct PlanView {
-    int nsn, max_m;
-    const int *col0, *ncol, *nrow, *parent;
+    int nsn, n_fwd, ntasks;
     const int* rows;
-    const long long* rows_off;
-    const int *child_ptr, *child;
-    const long long* relmap_off;
-    const int* relmap;
+    const int* child;
     // Gather lists: position p of front J's input vector receives the update
     // entries gent[ge_off[J] + gptr[gp_off[J] + p] .. gptr[gp_off[J] + p + 1])
     // (indices into upd), in child order.
-    const long long *gp_off, *ge_off;
     const int *gptr, *gent;
-    const long long* upd_off;
-    const long long* fw_off;
     const int *ntf, *ntb;
     const int* perm;
-    const int *bfwd, *bbwd;
     const float* fw;
+    const SnTask* tasks;
+    const float* b_old;
+    float* x_old;
     double* part;
     double* upd;
     double* ynew;
     double* xnew;
     int* ctr;
     int* err;
-    long long spin_limit;  // polls (with ~128 ns sleeps) before a wait gives up
-    // Right-hand side j (of K solved together) uses part + j ld_part,
-    // upd + j ld_upd, ynew / xnew + j ld_n, b_old + j ld_b, x_old + j ld_x.
-    long long ld_part, ld_upd, ld_n, ld_b, ld_x;
+    long long spin_limit;  // polls before a wait gives up
+    // Right-hand side j uses part + j ld_part, upd + j ld_upd, ynew / xnew + j
+    // ld_n, ctr + j ld_ctr (the ticket is shared), b_old + j ld_b, x_old + j ld_x.
+    long long ld_part, ld_upd, ld_n, ld_ctr, ld_b, ld_x;
+    int nrhs;
 };
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
@@ -108,20 +126,33 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
     asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ void add_release(int* p) {
+    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" : : "l"(p) : "memory");
+}
+__device__ __forceinline__ int add_acq_rel(int* p) {
+    int v;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 
-// Waits until *p >= target; false when the wait gave up, or at once when an
+// Waits until *p >= target; false when the wait gave up, or soon when an
 // earlier wait of this launch already gave up (so one failure cannot turn
 // into a long chain of timeouts).
-__device__ bool wait_at_least(const int* p, int target, const int* err, long long limit) {
+__device__ __noinline__ bool wait_at_least(const int* p, int target, const int* err, long long limit) {
     for (long long i = 0; i < limit; ++i) {
         if (ld_acquire(p) >= target) return true;
-        if (ld_acquire(err) != 0) return false;
-        __nanosleep(128);
+        if (i % 16 == 15 && ld_acquire(err) != 0) return false;
     }
     return false;
 }
 
 __device__ __forceinline__ float4 ldg4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+
+// Keeps v as FP32 up to here: converted to FP64 before a wait, the preloaded
+// coefficients would take twice the registers.
+__device__ __forceinline__ void hold(float4& v) {
+    asm volatile("" : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w));
+}
 
 // Four FP64 fused multiply-adds acc[e] += v.e * x.
 __device__ __forceinline__ void fma4(double (&acc)[4], const float4 v, double x) {
@@ -135,582 +166,360 @@ __device__ __forceinline__ void fma4(double (&acc)[4], const float4 v, double x)
 // columns starting on 16-byte boundaries, so four consecutive rows of a column
 // are one 16-byte load.  Entries above the diagonal of L_JJ^{-1} and the
 // padding rows m .. round4(m) are stored zeros: a load may cover them.
-//
-// K right-hand sides are solved together: each coefficient load feeds K
-// products.  A front's vectors in shared memory hold entry i of right-hand
-// side j at i * K + j.  Every right-hand side's arithmetic (which products,
-// summed in which order) is the same for every K, so a solve's result does not
-// depend on what it was batched with.
 
-// Forward solve of one small front by one warp: the lane owns the row quads
-// 4 * (lane + 32 q), q < MQ.
-template <int MQ, int K>
-__device__ __forceinline__ void warp_forward_rows(const PlanView& P, int J, int m, int nj, const double* f, int lane) {
-    const size_t ld = (size_t)((m + 3) & ~3);
-    const float* A = P.fw + P.fw_off[J];
-    double acc[MQ][K][4];
+// The vectors of one right-hand side.
+struct Vectors {
+    double *part, *upd, *y, *x;
+    int *done_f, *done_b, *chunk;
+    const float* b;
+    float* x_old;
+};
+
+struct Shared {
+    SnTask task[2];
+    Vectors vec[2];       // of the task's right-hand side (here to save registers)
+    int next[2];          // tickets of task[]
+    int last;
+    alignas(16) double f[kWhole];  // forward: the task's inputs
+    double fr[kRB];                // ... and its update rows' sums of the children's entries
+    double red[4 * kNT];           // column-slice partial sums; backward: the input rows
+};
+static_assert(4 * kNT >= rows_of(2), "backward inputs fit");
+
+template <class Fetch>
+__device__ __forceinline__ void forward_task(const PlanView& P, const SnTask& T, Shared& S, const Vectors& V,
+                                             Fetch fetch_next) {
+    const int tid = threadIdx.x, nj = T.nj;
+    // Row quads x column slices: mq lanes on the block's row quads (one
+    // 16-byte load per column), ks slices of consecutive columns.
+    const int nq = (T.rows + 3) >> 2;
+    const int mq = nq <= 8 ? 8 : (nq <= 16 ? 16 : 32);
+    const int ks = kNT / mq;
+    const int sl = tid / mq, lq = tid - sl * mq;
+    const int row = T.r0 + 4 * lq;
+    const size_t ld = (size_t)((T.m + 3) & ~3);
+    const float* A = P.fw + T.fw + row;
+    int cbeg = 0, cend = 0;
+    if (lq < nq) {
+        const int cs = (T.ncols + ks - 1) / ks;
+        cbeg = T.c0 + sl * cs;
+        cend = min(T.c0 + T.ncols, cbeg + cs);
+        if (row < nj) cend = min(cend, row + 4);  // L_JJ^{-1} is lower triangular
+    }
+    constexpr int U = 16;
+    float4 v[U];
+    const float* col = A + (size_t)cbeg * ld;
 #pragma unroll
-    for (int q = 0; q < MQ; ++q)
+    for (int u = 0; u < U; ++u) {
+        v[u] = (cbeg + u < cend) ? ldg4(col) : make_float4(0.f, 0.f, 0.f, 0.f);
+        col += ld;
+    }
+    // The positions this task reads, its columns and its update rows from
+    // max(r0, nj) on: b's entry and the gather indices now, the children's
+    // update entries after the wait.
+    const int rlo = max(T.r0, nj), rend = T.r0 + T.rows;
+    const int nneed = T.ncols + max(0, rend - rlo);
+    constexpr int Q = (kWhole + kRB + kNT - 1) / kNT;
+    double base[Q];
+    int e0[Q], e1[Q], first[Q], second[Q];
+    const bool kids = T.kids != 0;
 #pragma unroll
-        for (int j = 0; j < K; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[q][j][e] = 0.0;
-#pragma unroll 4
-    for (int c = 0; c < nj; ++c) {
-        double fc[K];
-#pragma unroll
-        for (int j = 0; j < K; ++j) fc[j] = f[(size_t)c * K + j];
-        const float* col = A + (size_t)c * ld;
-#pragma unroll
-        for (int q = 0; q < MQ; ++q) {
-            const int r = 4 * (lane + 32 * q);
-            if (r < m && r + 3 >= c) {
-                const float4 v = ldg4(col + r);
-#pragma unroll
-                for (int j = 0; j < K; ++j) fma4(acc[q][j], v, fc[j]);
+    for (int h = 0; h < Q; ++h) {
+        const int q = tid + h * kNT;
+        base[h] = 0.0;
+        e0[h] = e1[h] = first[h] = second[h] = 0;
+        if (q < nneed) {
+            const int p = q < T.ncols ? T.c0 + q : rlo + (q - T.ncols);
+            if (q < T.ncols) base[h] = (double)V.b[P.perm[T.col0 + p]];
+            if (kids) {
+                e0[h] = P.gptr[T.gp + p];
+                e1[h] = P.gptr[T.gp + p + 1];
+                if (e1[h] > e0[h]) first[h] = P.gent[T.ge + e0[h]];
+                if (e1[h] > e0[h] + 1) second[h] = P.gent[T.ge + e0[h] + 1];
             }
         }
     }
-    const int c0 = P.col0[J];
-    const long long uo = P.upd_off[J];
-#pragma unroll
-    for (int q = 0; q < MQ; ++q)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int r = 4 * (lane + 32 * q) + e;
-            if (r >= m) continue;
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                if (r < nj) P.ynew[j * P.ld_n + c0 + r] = acc[q][j][e];
-                else P.upd[j * P.ld_upd + uo + (r - nj)] = f[(size_t)r * K + j] + acc[q][j][e];
-            }
-        }
-}
-
-template <int K>
-__device__ void warp_forward(const PlanView& P, int J, double* f, int lane, const float* b_old, int* done) {
-    const int nj = P.ncol[J], m = nj + P.nrow[J], c0 = P.col0[J];
-    const int cb = P.child_ptr[J], ce = P.child_ptr[J + 1];
-    for (int i = lane; i < m; i += 32) {
-        const int po = i < nj ? P.perm[c0 + i] : 0;
-#pragma unroll
-        for (int j = 0; j < K; ++j) f[(size_t)i * K + j] = (i < nj) ? (double)b_old[j * P.ld_b + po] : 0.0;
-    }
-    if (lane == 0) {
+    if (kids && tid < 32) {
         bool ok = true;
-        for (int c = cb; c < ce; ++c) ok &= wait_at_least(done + P.child[c], P.ntf[P.child[c]], P.err, P.spin_limit);
+        for (int c = T.child_b + tid; c < T.child_e; c += 32) {
+            const int C = P.child[c];
+            ok &= wait_at_least(V.done_f + C, P.ntf[C], P.err, P.spin_limit);
+        }
         if (!ok) atomicExch(P.err, 1);
     }
-    __syncwarp();
-    for (int c = cb; c < ce; ++c) {
-        const int C = P.child[c];
-        const int mc = P.nrow[C];
-        const double* uc = P.upd + P.upd_off[C];
-        const int* rm = P.relmap + P.relmap_off[C];
-        for (int k = lane; k < mc; k += 32) {
-            const int t = rm[k];
+    fetch_next();
+    __syncthreads();
+    double u0[Q], u1[Q];
 #pragma unroll
-            for (int j = 0; j < K; ++j) f[(size_t)t * K + j] += __ldcg(uc + j * P.ld_upd + k);
-        }
-        __syncwarp();
+    for (int h = 0; h < Q; ++h) {
+        u0[h] = e1[h] > e0[h] ? __ldcg(V.upd + first[h]) : 0.0;
+        u1[h] = e1[h] > e0[h] + 1 ? __ldcg(V.upd + second[h]) : 0.0;
     }
-    if (m <= 128) warp_forward_rows<1, K>(P, J, m, nj, f, lane);
-    else warp_forward_rows<2, K>(P, J, m, nj, f, lane);
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) atomicAdd(done + J, 1);
+#pragma unroll
+    for (int h = 0; h < Q; ++h) {
+        const int q = tid + h * kNT;
+        if (q >= nneed) continue;
+        double s = base[h] + u0[h] + u1[h];
+        for (int e = e0[h] + 2; e < e1[h]; ++e) s += __ldcg(V.upd + P.gent[T.ge + e]);
+        if (q < T.ncols) S.f[q] = s;
+        else S.fr[rlo + (q - T.ncols) - T.r0] = s;
+    }
+    __syncthreads();
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const double* f = S.f - T.c0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        hold(v[u]);
+        if (cbeg + u < cend) fma4(acc, v[u], f[cbeg + u]);
+    }
+    for (int c = cbeg + U; c < cend; c += 8) {
+        float4 w[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            w[u] = (c + u < cend) ? ldg4(col) : make_float4(0.f, 0.f, 0.f, 0.f);
+            col += ld;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (c + u < cend) fma4(acc, w[u], f[c + u]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) S.red[e * kNT + tid] = acc[e];
+    __syncthreads();
+    // Thread t < rows adds row r0 + t's slices in order.
+    const int r = T.r0 + tid;
+    double s = 0.0;
+    if (tid < T.rows) {
+        const double* p = S.red + (tid & 3) * kNT + (tid >> 2);
+        s = p[0];
+#pragma unroll 8
+        for (int q = 1; q < ks; ++q) s += p[q * mq];
+    }
+    if (T.nk > 1) {
+        if (tid < T.rows) V.part[T.part + (size_t)T.k * kRB + tid] = s;
+        __syncthreads();
+        if (tid == 0) S.last = add_acq_rel(V.chunk + T.chunk) == T.nk - 1;
+        __syncthreads();
+        if (S.last && tid < T.rows) {
+            s = 0.0;
+            for (int k = 0; k < T.nk; ++k) s += __ldcg(V.part + T.part + (size_t)k * kRB + tid);
+        }
+    }
+    if (tid < T.rows && (T.nk == 1 || S.last)) {
+        if (r < nj) V.y[T.col0 + r] = s;
+        else V.upd[T.upd + (r - nj)] = S.fr[tid] + s;
+    }
+    __syncthreads();
+    if (tid == 0) add_release(V.done_f + T.front);
 }
 
-// Backward solve of one small front by one warp: x_a = sum_{r >= a} Fw(r, a) g_r,
-// four columns at a time, the lane summing the row quads a + 4 lane + 128 k.
-template <int K>
-__device__ void warp_backward(const PlanView& P, int J, double* g, int lane, float* x_old, int* done) {
-    const int nj = P.ncol[J], m = nj + P.nrow[J], c0 = P.col0[J];
-    const int m4 = (m + 3) & ~3;
-    const int* rows = P.rows + P.rows_off[J];
-    for (int i = lane; i < nj; i += 32)  // from the forward launch
+// CW columns per warp.
+template <int CW, class Fetch>
+__device__ __forceinline__ void backward_task(const PlanView& P, const SnTask& T, Shared& S, const Vectors& V,
+                                              Fetch fetch_next) {
+    constexpr int NI = kBLoads / CW, Q = rows_of(CW) / kNT;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nj = T.nj;
+    // Columns [r0, r0 + rows) of the front; this task's rows [rlo, rhi): all
+    // from r0 on (the first any of its columns needs, a multiple of 4), or one
+    // chunk of them.
+    const int a0 = T.r0, na = T.rows, rlo = T.c0, rhi = T.c0 + T.ncols;
+    const size_t ld = (size_t)((T.m + 3) & ~3);
+    const float* A = P.fw + T.fw;
+    double* g = S.red;  // input rows, entry i - rlo
+    float4 v[NI][CW];
+    const float* col = A + (size_t)(a0 + w) * ld + rlo + 4 * lane;
 #pragma unroll
-        for (int j = 0; j < K; ++j) g[(size_t)i * K + j] = P.ynew[j * P.ld_n + c0 + i];
-    for (int i = m + lane; i < m4; i += 32)  // padding rows
+    for (int j = 0; j < CW; ++j) {
+        const bool on = w + kWarps * j < na;
 #pragma unroll
-        for (int j = 0; j < K; ++j) g[(size_t)i * K + j] = 0.0;
+        for (int i = 0; i < NI; ++i)
+            v[i][j] = (on && rlo + 4 * lane + 128 * i < rhi) ? ldg4(col + 128 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        col += kWarps * ld;
+    }
+    int src[Q];
+#pragma unroll
+    for (int h = 0; h < Q; ++h) {
+        const int i = rlo + tid + h * kNT;
+        src[h] = (i >= nj && i < rhi) ? P.rows[T.rows_off + (i - nj)] : 0;
+    }
+    if (tid == 0) {
+        // The parent's solution, or (at a root) this front's forward result.
+        const bool root = T.parent < 0;
+        const int* d = root ? V.done_f + T.front : V.done_b + T.parent;
+        const int target = root ? P.ntf[T.front] : P.ntb[T.parent];
+        if (!wait_at_least(d, target, P.err, P.spin_limit)) atomicExch(P.err, 1);
+    }
+    fetch_next();
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < Q; ++h) {
+        const int i = rlo + tid + h * kNT;
+        if (i < nj && i < rhi) g[i - rlo] = __ldcg(V.y + T.col0 + i);
+        else if (i < rhi) g[i - rlo] = __ldcg(V.x + src[h]);
+        else if (i < rlo + rows_of(CW)) g[i - rlo] = 0.0;  // padding rows
+    }
+    __syncthreads();
+    double s[CW];
+#pragma unroll
+    for (int j = 0; j < CW; ++j) s[j] = 0.0;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int q = 4 * lane + 128 * i;
+        if (rlo + q >= rhi) continue;
+        const double2 g0 = *reinterpret_cast<const double2*>(g + q), g1 = *reinterpret_cast<const double2*>(g + q + 2);
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+            hold(v[i][j]);
+            s[j] = fma((double)v[i][j].x, g0.x, s[j]);
+            s[j] = fma((double)v[i][j].y, g0.y, s[j]);
+            s[j] = fma((double)v[i][j].z, g1.x, s[j]);
+            s[j] = fma((double)v[i][j].w, g1.y, s[j]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < CW; ++j)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+    auto write_x = [&](int a, double x) {
+        V.x[T.col0 + a] = x;
+        V.x_old[P.perm[T.col0 + a]] = (float)x;
+    };
     if (lane == 0) {
-        const int p = P.parent[J];
-        if (p >= 0 && !wait_at_least(done + p, P.ntb[p], P.err, P.spin_limit)) atomicExch(P.err, 1);
-    }
-    __syncwarp();
-    for (int i = nj + lane; i < m; i += 32) {
-        const int t = rows[i - nj];
 #pragma unroll
-        for (int j = 0; j < K; ++j) g[(size_t)i * K + j] = __ldcg(P.xnew + j * P.ld_n + t);
-    }
-    __syncwarp();
-    const size_t ld = (size_t)m4;
-    const float* A = P.fw + P.fw_off[J];
-    for (int a = 0; a < nj; a += 4) {
-        double s4[K][4];
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) s4[j][jj] = 0.0;
-#pragma unroll 2
-        for (int r = a + 4 * lane; r < m; r += 128) {
-            double gg[K][4];
-#pragma unroll
-            for (int j = 0; j < K; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) gg[j][e] = g[(size_t)(r + e) * K + j];
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
-                if (a + jj < nj) {
-                    const float4 v = ldg4(A + (size_t)(a + jj) * ld + r);
-#pragma unroll
-                    for (int j = 0; j < K; ++j) {
-                        s4[j][jj] = fma((double)v.x, gg[j][0], s4[j][jj]);
-                        s4[j][jj] = fma((double)v.y, gg[j][1], s4[j][jj]);
-                        s4[j][jj] = fma((double)v.z, gg[j][2], s4[j][jj]);
-                        s4[j][jj] = fma((double)v.w, gg[j][3], s4[j][jj]);
-                    }
-                }
-        }
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s4[j][jj] += __shfl_xor_sync(0xffffffffu, s4[j][jj], o);
-        if (lane == 0) {
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
-                if (a + jj < nj) {
-                    const int po = P.perm[c0 + a + jj];
-#pragma unroll
-                    for (int j = 0; j < K; ++j) {
-                        P.xnew[j * P.ld_n + c0 + a + jj] = s4[j][jj];
-                        x_old[j * P.ld_x + po] = (float)s4[j][jj];
-                    }
-                }
+        for (int j = 0; j < CW; ++j) {
+            const int a = a0 + w + kWarps * j;
+            if (a >= a0 + na) continue;
+            if (T.nk == 1) write_x(a, s[j]);
+            else V.part[T.part + (size_t)T.k * cols_of(CW) + (a - a0)] = s[j];
         }
     }
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) atomicAdd(done + J, 1);
+    __syncthreads();
+    if (T.nk > 1) {
+        if (tid == 0) S.last = add_acq_rel(V.chunk + T.chunk) == T.nk - 1;
+        __syncthreads();
+        if (S.last && tid < na) {
+            double x = 0.0;
+            for (int k = 0; k < T.nk; ++k) x += __ldcg(V.part + T.part + (size_t)k * cols_of(CW) + tid);
+            write_x(a0 + tid, x);
+        }
+        __syncthreads();
+    }
+    if (tid == 0) add_release(V.done_b + T.front);
 }
 
-template <int K, int NT>
-__global__ void __launch_bounds__(NT, min_blocks(K, NT))
-    sn_forward_kernel(PlanView P, const SnTask* __restrict__ tasks, int ntasks, const float* __restrict__ b_old) {
-    extern __shared__ double sh[];
-    double* f = sh;                    // the front's input vectors, m x K entries
-    double* red = sh + P.max_m * K;    // column-slice partial sums, 4 K NT entries
-    __shared__ int s_ticket, s_last;
-    int* done = P.ctr + 2;
-    int* chunk_ctr = P.ctr + 2 + 2 * P.nsn;
-    const int tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) s_ticket = atomicAdd(P.ctr + 0, 1);
-        __syncthreads();
-        const int t = s_ticket;
-        if (t >= ntasks) break;
-        const SnTask T = tasks[t];
-        if (T.front < 0) {
-            const int w = tid >> 5;
-            if (w < T.rows) warp_forward<K>(P, P.bfwd[T.r0 + w], sh + (size_t)w * kSmallM * K, tid & 31, b_old, done);
-            __syncthreads();
-            continue;
+__global__ void __launch_bounds__(kNT, kPerSM) sn_task_kernel(PlanView P) {
+    __shared__ __align__(16) Shared S;
+    const int tid = threadIdx.x, total = P.ntasks * P.nrhs;
+    // One warp fetches a ticket and its task's record.
+    auto fetch = [&](int slot) {
+        int t = 0;
+        if ((tid & 31) == 0) t = atomicAdd(P.ctr, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if ((tid & 31) == 0) {
+            S.next[slot] = t;
+            const int j = t % P.nrhs;
+            int* ctr = P.ctr + 1 + j * P.ld_ctr;
+            S.vec[slot] = {P.part + j * P.ld_part, P.upd + j * P.ld_upd, P.ynew + j * P.ld_n, P.xnew + j * P.ld_n,
+                           ctr, ctr + P.nsn, ctr + 2 * P.nsn, P.b_old + j * P.ld_b, P.x_old + j * P.ld_x};
         }
-        const int J = T.front, nj = P.ncol[J], m = nj + P.nrow[J], c0 = P.col0[J];
-        const int cb = P.child_ptr[J], ce = P.child_ptr[J + 1];
-        // Row quads x column slices: the block's rows in quads of four (one
-        // 16-byte load per column), mq quad lanes per slice, ks slices.  Each
-        // thread's first four coefficient loads are issued before the
-        // dependency wait and the assembly.
-        const int nq = (T.rows + 3) >> 2;
-        const int mq = nq <= 8 ? 8 : (nq <= 16 ? 16 : 32);
-        const int ks = NT / mq;
-        const int sl = tid / mq, lq = tid - sl * mq;
-        const int row = T.r0 + 4 * lq;
-        const bool active = lq < nq;
-        int cbeg = 0, cend = 0;
-        const size_t ld = (size_t)((m + 3) & ~3);
-        const float* A = P.fw + P.fw_off[J] + row;
-        if (active) {
-            const int cs = (T.ncols + ks - 1) / ks;
-            cbeg = T.c0 + sl * cs;
-            cend = min(T.c0 + T.ncols, cbeg + cs);
-            if (row < nj) cend = min(cend, row + 4);  // L_JJ^{-1} is lower triangular
-        }
-        float4 v0[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            v0[u] = (cbeg + u < cend) ? ldg4(A + (size_t)(cbeg + u) * ld) : make_float4(0.f, 0.f, 0.f, 0.f);
-        if constexpr (NT < 128) {
-            // Small fronts (the interior plans' 64-thread CTAs): the whole
-            // input vectors, b's part before the wait, then each child's
-            // update scattered in, child by child.
-            for (int i = tid; i < m; i += NT) {
-                const int po = i < nj ? P.perm[c0 + i] : 0;
-#pragma unroll
-                for (int j = 0; j < K; ++j) f[(size_t)i * K + j] = (i < nj) ? (double)b_old[j * P.ld_b + po] : 0.0;
-            }
-            if (tid == 0) {
-                bool ok = true;
-                for (int c = cb; c < ce; ++c)
-                    ok &= wait_at_least(done + P.child[c], P.ntf[P.child[c]], P.err, P.spin_limit);
-                if (!ok) atomicExch(P.err, 1);
-            }
-            __syncthreads();
-            for (int c = cb; c < ce; ++c) {
-                const int C = P.child[c];
-                const int mc = P.nrow[C];
-                const double* uc = P.upd + P.upd_off[C];
-                const int* rm = P.relmap + P.relmap_off[C];
-                for (int k = tid; k < mc; k += NT) {
-                    const int tr = rm[k];
-#pragma unroll
-                    for (int j = 0; j < K; ++j) f[(size_t)tr * K + j] += __ldcg(uc + j * P.ld_upd + k);
-                }
-                __syncthreads();
-            }
-        } else {
-            // Tall fronts (the interface plans): only the positions this task
-            // reads, its columns [T.c0, T.c0 + T.ncols) and its update rows
-            // [max(T.r0, nj), rend); b's part before the wait, then each
-            // position adds its children's update entries in child order,
-            // the same sums as the whole-front scatter above.  Measured: the
-            // level-0 interface forward drops from 485 to 436 us.
-            const int rlo = max(T.r0, nj), nrn = max(0, T.r0 + T.rows - rlo);
-            const int nneed = T.ncols + nrn;
-            for (int q = tid; q < nneed; q += NT) {
-                const int p = q < T.ncols ? T.c0 + q : rlo + (q - T.ncols);
-                const int po = p < nj ? P.perm[c0 + p] : 0;
-#pragma unroll
-                for (int j = 0; j < K; ++j) f[(size_t)p * K + j] = (p < nj) ? (double)b_old[j * P.ld_b + po] : 0.0;
-            }
-            if (tid == 0) {
-                bool ok = true;
-                for (int c = cb; c < ce; ++c)
-                    ok &= wait_at_least(done + P.child[c], P.ntf[P.child[c]], P.err, P.spin_limit);
-                if (!ok) atomicExch(P.err, 1);
-            }
-            __syncthreads();
-            if (ce > cb) {
-                const int* gp = P.gptr + P.gp_off[J];
-                const int* ge = P.gent + P.ge_off[J];
-                for (int q = tid; q < nneed; q += NT) {
-                    const int p = q < T.ncols ? T.c0 + q : rlo + (q - T.ncols);
-                    double v[K];
-#pragma unroll
-                    for (int j = 0; j < K; ++j) v[j] = f[(size_t)p * K + j];
-                    for (int e = gp[p]; e < gp[p + 1]; ++e) {
-                        const int ui = ge[e];
-#pragma unroll
-                        for (int j = 0; j < K; ++j) v[j] += __ldcg(P.upd + j * P.ld_upd + ui);
-                    }
-#pragma unroll
-                    for (int j = 0; j < K; ++j) f[(size_t)p * K + j] = v[j];
-                }
-                __syncthreads();
-            }
-        }
-        double acc[K][4];
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[j][e] = 0.0;
-        if (active) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (cbeg + u < cend)
-#pragma unroll
-                    for (int j = 0; j < K; ++j) fma4(acc[j], v0[u], f[(size_t)(cbeg + u) * K + j]);
-            int c = cbeg + 4;
-            for (; c + 4 <= cend; c += 4) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) v0[u] = ldg4(A + (size_t)(c + u) * ld);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int j = 0; j < K; ++j) fma4(acc[j], v0[u], f[(size_t)(c + u) * K + j]);
-            }
-            for (; c < cend; ++c) {
-                const float4 v = ldg4(A + (size_t)c * ld);
-#pragma unroll
-                for (int j = 0; j < K; ++j) fma4(acc[j], v, f[(size_t)c * K + j]);
-            }
-        }
-        if (ks > 1) {
-#pragma unroll
-            for (int j = 0; j < K; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) red[(size_t)(j * 4 + e) * NT + tid] = acc[j][e];
-            __syncthreads();
-            if (sl == 0 && active) {
-#pragma unroll
-                for (int j = 0; j < K; ++j)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        double s2 = red[(size_t)(j * 4 + e) * NT + lq];
-                        for (int q = 1; q < ks; ++q) s2 += red[(size_t)(j * 4 + e) * NT + q * mq + lq];
-                        acc[j][e] = s2;
-                    }
-            }
-        }
-        const bool mine = sl == 0 && active;
-        const int rend = T.r0 + T.rows;
-        if (T.nk == 1) {
-            if (mine) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = row + e;
-                    if (r >= rend) break;
-#pragma unroll
-                    for (int j = 0; j < K; ++j) {
-                        if (r < nj) P.ynew[j * P.ld_n + c0 + r] = acc[j][e];
-                        else P.upd[j * P.ld_upd + P.upd_off[J] + (r - nj)] = f[(size_t)r * K + j] + acc[j][e];
-                    }
-                }
-            }
-        } else {
-            if (mine) {
-#pragma unroll
-                for (int j = 0; j < K; ++j) {
-                    double* pp = P.part + j * P.ld_part + T.part + (size_t)T.k * kRB + 4 * lq;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) pp[e] = acc[j][e];
-                }
-            }
-            __threadfence();
-            __syncthreads();
-            if (tid == 0) s_last = (atomicAdd(chunk_ctr + T.chunk, 1) == T.nk - 1);
-            __syncthreads();
-            if (s_last) {
-                __threadfence();
-                if (mine) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int r = row + e;
-                        if (r >= rend) break;
-#pragma unroll
-                        for (int j = 0; j < K; ++j) {
-                            const double* pj = P.part + j * P.ld_part + T.part + 4 * lq + e;
-                            double s2 = 0.0;
-                            for (int k = 0; k < T.nk; ++k) s2 += __ldcg(pj + (size_t)k * kRB);
-                            if (r < nj) P.ynew[j * P.ld_n + c0 + r] = s2;
-                            else P.upd[j * P.ld_upd + P.upd_off[J] + (r - nj)] = f[(size_t)r * K + j] + s2;
-                        }
-                    }
-                }
-            }
-        }
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) atomicAdd(done + J, 1);
-    }
-}
-
-template <int K, int NT>
-__global__ void __launch_bounds__(NT, min_blocks(K, NT))
-    sn_backward_kernel(PlanView P, const SnTask* __restrict__ tasks, int ntasks, float* __restrict__ x_old) {
-    extern __shared__ double g[];  // [y_J; x_R] x K, m4 x K entries (zero padding rows)
-    __shared__ int s_ticket, s_last;
-    int* done = P.ctr + 2 + P.nsn;
-    int* chunk_ctr = P.ctr + 2 + 2 * P.nsn;
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    for (;;) {
-        if (tid == 0) s_ticket = atomicAdd(P.ctr + 1, 1);
-        __syncthreads();
-        const int t = s_ticket;
-        if (t >= ntasks) break;
-        const SnTask T = tasks[t];
-        if (T.front < 0) {
-            if (w < T.rows) warp_backward<K>(P, P.bbwd[T.r0 + w], g + (size_t)w * kSmallM * K, lane, x_old, done);
-            __syncthreads();
-            continue;
-        }
-        const int J = T.front, nj = P.ncol[J], m = nj + P.nrow[J], c0 = P.col0[J];
-        const int m4 = (m + 3) & ~3;
-        const int a0 = T.r0, na = T.rows;
-        // This task's rows [rlo, rhi): all rows from a0 (the first any of its
-        // columns needs, a multiple of 4), or one chunk of them when a tall
-        // column block is split (chunks start at multiples of 4; partial sums
-        // of the chunks are added in chunk order by the last one to finish).
-        const int rlo = T.c0, rhi = T.c0 + T.ncols;
-        const int* rows = P.rows + P.rows_off[J];
-        const size_t ld = (size_t)m4;
-        const float* A = P.fw + P.fw_off[J];
-        double s4[K][4];
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) s4[j][jj] = 0.0;
-        const int amin = a0 + w;
-        // Row quads wholly below nj (the L_JJ^{-T} y part) need only this
-        // front's forward result, so they are summed before waiting on the
-        // parent; each lane adds its quads in ascending order.
-        const int yhi = min(rhi, nj);
-        for (int i = rlo + tid; i < yhi; i += NT)  // from the forward launch
-#pragma unroll
-            for (int j = 0; j < K; ++j) g[(size_t)i * K + j] = P.ynew[j * P.ld_n + c0 + i];
-        if (rhi == m)
-            for (int i = m + tid; i < m4; i += NT)  // padding rows
-#pragma unroll
-                for (int j = 0; j < K; ++j) g[(size_t)i * K + j] = 0.0;
-        __syncthreads();
-        int r = rlo + 4 * lane;
-        auto quad = [&](int rr) {
-            double gg[K][4];
-#pragma unroll
-            for (int j = 0; j < K; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) gg[j][e] = g[(size_t)(rr + e) * K + j];
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const int a = amin + warps_of(NT) * jj;
-                if (a < a0 + na) {
-                    const float4 v = ldg4(A + (size_t)a * ld + rr);
-#pragma unroll
-                    for (int j = 0; j < K; ++j) {
-                        s4[j][jj] = fma((double)v.x, gg[j][0], s4[j][jj]);
-                        s4[j][jj] = fma((double)v.y, gg[j][1], s4[j][jj]);
-                        s4[j][jj] = fma((double)v.z, gg[j][2], s4[j][jj]);
-                        s4[j][jj] = fma((double)v.w, gg[j][3], s4[j][jj]);
-                    }
-                }
-            }
+        constexpr int N4 = (int)(sizeof(SnTask) / sizeof(int4));
+        if (t < total && (tid & 31) < N4)
+            reinterpret_cast<int4*>(&S.task[slot])[tid & 31] =
+                __ldg(reinterpret_cast<const int4*>(P.tasks + t / P.nrhs) + (tid & 31));
+    };
+    if (tid < 32) fetch(0);
+    __syncthreads();
+    for (int cur = 0;; cur ^= 1) {
+        const int t = S.next[cur];
+        if (t >= total) break;
+        // The last warp fetches the next task once this one's loads are issued.
+        auto fetch_next = [&]() {
+            if (tid >= kNT - 32) fetch(cur ^ 1);
         };
-        if (amin < a0 + na) {
-#pragma unroll 2
-            for (; r + 4 <= yhi; r += 128) quad(r);
-        }
-        if (rhi > nj) {
-            // The update rows need the parent's solution.
-            if (tid == 0) {
-                const int p = P.parent[J];
-                if (p >= 0 && !wait_at_least(done + p, P.ntb[p], P.err, P.spin_limit)) atomicExch(P.err, 1);
-            }
-            __syncthreads();
-            for (int i = max(rlo, nj) + tid; i < rhi; i += NT) {
-                const int tr = rows[i - nj];
-#pragma unroll
-                for (int j = 0; j < K; ++j) g[(size_t)i * K + j] = __ldcg(P.xnew + j * P.ld_n + tr);
-            }
-            __syncthreads();
-        }
-        // The rest: the update rows, and the quad that straddles nj (its rows
-        // past m are the zero padding).
-        if (amin < a0 + na) {
-#pragma unroll 2
-            for (; r < rhi; r += 128) quad(r);
-        }
-#pragma unroll
-        for (int j = 0; j < K; ++j)
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj)
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s4[j][jj] += __shfl_xor_sync(0xffffffffu, s4[j][jj], o);
-        auto write_x = [&](int a, int j, double v) {
-            P.xnew[j * P.ld_n + c0 + a] = v;
-            x_old[j * P.ld_x + P.perm[c0 + a]] = (float)v;
-        };
-        if (T.nk == 1) {
-            if (lane == 0) {
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    const int a = amin + warps_of(NT) * jj;
-                    if (a < a0 + na)
-#pragma unroll
-                        for (int j = 0; j < K; ++j) write_x(a, j, s4[j][jj]);
-                }
-            }
-        } else {
-            // Partial sums of this chunk: column (a - a0) of chunk k.
-            if (lane == 0) {
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    const int a = amin + warps_of(NT) * jj;
-                    if (a < a0 + na)
-#pragma unroll
-                        for (int j = 0; j < K; ++j)
-                            P.part[j * P.ld_part + T.part + (size_t)T.k * bc_of(NT) + (a - a0)] = s4[j][jj];
-                }
-            }
-            __threadfence();
-            __syncthreads();
-            if (tid == 0) s_last = (atomicAdd(chunk_ctr + T.chunk, 1) == T.nk - 1);
-            __syncthreads();
-            if (s_last) {
-                __threadfence();
-                for (int q = tid; q < na * K; q += NT) {
-                    const int c = q / K, j = q - c * K;
-                    const double* pj = P.part + j * P.ld_part + T.part + c;
-                    double v = 0.0;
-                    for (int k = 0; k < T.nk; ++k) v += __ldcg(pj + (size_t)k * bc_of(NT));
-                    write_x(a0 + c, j, v);
-                }
-            }
-        }
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) atomicAdd(done + J, 1);
+        const SnTask& T = S.task[cur];
+        const Vectors& V = S.vec[cur];
+        if (t / P.nrhs < P.n_fwd) forward_task(P, T, S, V, fetch_next);
+        else if (T.cw == 4) backward_task<4>(P, T, S, V, fetch_next);
+        else backward_task<2>(P, T, S, V, fetch_next);
+        __syncthreads();  // the records and inputs are reused
     }
 }
 
-size_t forward_smem(int max_m, int k, int nt) {
-    return (size_t)std::max((max_m + 4 * nt) * k, warps_of(nt) * kSmallM * k) * sizeof(double);
+double front_weight(const SnFactor& F, size_t j) {
+    return 1000.0 + 0.5 * F.ncol[j] * (F.ncol[j] + 1.0) + (double)F.rows[j].size() * F.ncol[j];
 }
-size_t backward_smem(int max_m, int k, int nt) {
-    return (size_t)std::max(((max_m + 3) & ~3) * k, warps_of(nt) * kSmallM * k) * sizeof(double);
-}
-
-// Right-hand-side counts a launch can take (template instances), and the
-// shared memory any of them may use.
-constexpr int kBatches[3] = {1, 2, 4};
-constexpr size_t kSmemMax = 227 * 1024;
-
-// The dynamic shared-memory limit of each kernel instance only ever grows,
-// so a plan built later with smaller fronts cannot invalidate an earlier
-// plan's launches.
-std::mutex g_smem_mu;
-int g_smem_limit[64][6] = {};
-template <int K, int NT>
-void raise_limit_k(int device, int bytes, int slot) {
-    if (bytes <= g_smem_limit[device][slot]) return;
-    dev::ck(cudaFuncSetAttribute(sn_forward_kernel<K, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-            "smem attr");
-    dev::ck(cudaFuncSetAttribute(sn_backward_kernel<K, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-            "smem attr");
-    g_smem_limit[device][slot] = bytes;
-}
-template <int NT>
-void raise_limit_nt(int device, int k, int bytes, int base) {
-    if (k == 1) raise_limit_k<1, NT>(device, bytes, base);
-    else if (k == 2) raise_limit_k<2, NT>(device, bytes, base + 1);
-    else raise_limit_k<4, NT>(device, bytes, base + 2);
-}
-void raise_smem_limit(int device, int k, int nt, int bytes) {
-    std::lock_guard<std::mutex> lock(g_smem_mu);
-    if (device < 0 || device >= 64) throw Error(HDD_ERR_INVALID_ARGUMENT, "device ordinal out of range");
-    if (nt == kNTInterior) raise_limit_nt<kNTInterior>(device, k, bytes, 0);
-    else raise_limit_nt<kNTInterface>(device, k, bytes, 3);
+double tree_weight(const SnFactor& F) {
+    double w = 0;
+    for (size_t j = 0; j < F.col0.size(); ++j) w += front_weight(F, j);
+    return w;
 }
 
-template <int K, int NT>
-int occupancy_k(size_t smf, size_t smb) {
-    int bf = 0, bb = 0;
-    dev::ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bf, sn_forward_kernel<K, NT>, NT, smf), "occupancy");
-    dev::ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bb, sn_backward_kernel<K, NT>, NT, smb), "occupancy");
-    return std::max(1, std::min(bf, bb));
+// Plans solved by one CTA per factor (sn_resident.cu): every factor's unknowns
+// fit a CTA's shared memory, and cutting them would not pay.
+bool resident_plan(const std::vector<const SnFactor*>& factors, double total) {
+    int max_n = 0;
+    double largest = 0;
+    for (const SnFactor* F : factors) {
+        max_n = std::max(max_n, F->n);
+        largest = std::max(largest, tree_weight(*F));
+    }
+    if (max_n == 0 || ResidentPlan::smem_bytes(max_n + kPartMax, 1, 512) > ResidentPlan::kMaxSmem) return false;
+    return largest <= kCutCost + total / kCutRate;
 }
-template <int NT>
-int occupancy_nt(int k, size_t smf, size_t smb) {
-    return k == 1 ? occupancy_k<1, NT>(smf, smb) : (k == 2 ? occupancy_k<2, NT>(smf, smb) : occupancy_k<4, NT>(smf, smb));
+
+// The lower trees of factor F (unknowns from `off` on, fronts from `base` on in
+// the plan): the largest subtrees of at most weight `cap`, each marked in low /
+// cut_root; consecutive ones share a CTA up to that weight.
+void cut_trees(const SnFactor& F, int off, int base, double cap, std::vector<char>& low, std::vector<char>& cut_root,
+               std::vector<ResidentPlan::Shape>& shapes, std::vector<int>& shape_off,
+               std::vector<std::vector<int>>& shape_roots) {
+    const int ns = (int)F.col0.size();
+    std::vector<double> weight(ns);
+    std::vector<int> size(ns, 1), len(ns);
+    for (int j = 0; j < ns; ++j) {
+        weight[j] += front_weight(F, j);
+        len[j] += F.ncol[j];
+        if (F.parent[j] >= 0) {
+            weight[F.parent[j]] += weight[j];
+            size[F.parent[j]] += size[j];
+            len[F.parent[j]] += len[j];
+        }
+    }
+    auto fits = [&](int j) { return weight[j] <= cap && (len[j] + (int)F.rows[j].size()) <= kCutLen; };
+    double w = 0;
+    int n = 0;
+    for (int j = 0; j < ns; ++j) {
+        if (!fits(j) || (F.parent[j] >= 0 && fits(F.parent[j]))) continue;
+        const int vec = len[j] + (int)F.rows[j].size();
+        if (shape_off.empty() || shapes.back().F != &F || shape_off.back() != off || w + weight[j] > cap ||
+            n + vec > kCutLen) {
+            shapes.emplace_back();
+            shapes.back().F = &F;
+            shapes.back().ext_off = off;
+            shape_off.push_back(off);
+            shape_roots.emplace_back();
+            w = 0;
+            n = 0;
+        }
+        w += weight[j];
+        n += vec;
+        shapes.back().trees.push_back({j - size[j] + 1, j, -1});
+        shape_roots.back().push_back(base + j);
+        cut_root[base + j] = 1;
+        for (int i = j - size[j] + 1; i <= j; ++i) low[base + i] = 1;
+    }
 }
 
 }  // namespace
 
+// Most unknowns a front above the trees may have rows and columns: each
+// right-hand side of a batch needs the vectors of the plan's largest front.
+size_t front_bytes(int max_front, int k) { return (size_t)(max_front + 4 * kNT) * k * sizeof(double); }
+constexpr size_t kSmemMax = 227 * 1024;
+constexpr size_t kFrontMax = 200 * 1024;
+
 void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s,
-                      int* shared_err) {
+                      int* shared_err, double shrink) {
     release();
     const bool verbose = std::getenv("HDD_VERBOSE") != nullptr;
     const auto t_start = std::chrono::steady_clock::now();
@@ -719,386 +528,316 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
             std::fprintf(stderr, "[hdd setup]   plan (%zu factors): %s at %.3f s\n", factors.size(), what,
                          std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count());
     };
-    std::vector<int> col0, ncol, nrow, rows, child_ptr{0}, child, relmap, perm, height, depth, parent_g;
-    std::vector<long long> rows_off, relmap_off, upd_off, fw_off;
-    n = 0;
-    for (size_t f = 0; f < factors.size(); ++f) n = std::max(n, offsets[f] + factors[f]->n);
-    perm.assign(n, 0);
-    std::vector<int> base(factors.size() + 1, 0);
-    for (size_t f = 0; f < factors.size(); ++f) base[f + 1] = base[f] + (int)factors[f]->col0.size();
-    nsn = base.back();
-    parent_g.assign(nsn, -1);
-    std::vector<std::vector<int>> kids(nsn);
-    std::vector<std::pair<int, int>> where(nsn);
-    for (size_t f = 0; f < factors.size(); ++f) {
-        const SnFactor& F = *factors[f];
-        if (F.Fw.size() != F.col0.size()) throw Error(HDD_ERR_INTERNAL, "solve blocks not built");
-        const int off = offsets[f];
-        for (int i = 0; i < F.n; ++i) perm[off + i] = off + F.perm[i];
-        for (size_t j = 0; j < F.col0.size(); ++j) {
-            const int g = base[f] + (int)j;
-            where[g] = {(int)f, (int)j};
-            if (F.parent[j] >= 0) {
-                parent_g[g] = base[f] + F.parent[j];
-                kids[parent_g[g]].push_back(g);
-            }
-        }
-    }
-    if (nsn == 0) return;
-    nt = factors.size() >= 2 ? kNTInterior : kNTInterface;
-    const int kWarps = warps_of(nt), kBC = bc_of(nt);
-    // Rows per backward task: about 16K coefficients per task, as a forward
-    // task's 128 x 128 block (512 rows of 32 columns, 2048 of 8).
-    const int kBRows = 16384 / kBC;
-    height.assign(nsn, 0);
-    depth.assign(nsn, 0);
-    for (int g = 0; g < nsn; ++g)
-        if (parent_g[g] >= 0) height[parent_g[g]] = std::max(height[parent_g[g]], height[g] + 1);
-    for (int g = nsn - 1; g >= 0; --g)
-        if (parent_g[g] >= 0) depth[g] = depth[parent_g[g]] + 1;
-    long long upd_total = 0, fw_total = 0;
-    max_front = 0;
-    for (int g = 0; g < nsn; ++g) {
-        const SnFactor& F = *factors[where[g].first];
-        const int j = where[g].second, off = offsets[where[g].first];
-        const int nj = F.ncol[j], nr = (int)F.rows[j].size(), m = nj + nr;
-        col0.push_back(off + F.col0[j]);
-        ncol.push_back(nj);
-        nrow.push_back(nr);
-        max_front = std::max(max_front, m);
-        rows_off.push_back((long long)rows.size());
-        for (int r : F.rows[j]) rows.push_back(off + r);
-        upd_off.push_back(upd_total);
-        upd_total += nr;
-        fw_off.push_back(fw_total);
-        fw_total += (long long)((m + 3) & ~3) * nj;
-    }
-    // Tasks in topological order.
-    std::vector<int> order(nsn);
-    for (int g = 0; g < nsn; ++g) order[g] = g;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return height[a] < height[b]; });
-    std::vector<SnTask> ftasks, btasks;
-    std::vector<int> ntf(nsn, 0), ntb(nsn, 0), bfwd, bbwd;
-    int nchunk = 0;
-    long long part_total = 0;
-    // Small fronts of one level go in bundles of kWarps, one warp each.
-    auto flush = [](std::vector<SnTask>& tasks, std::vector<int>& list, int& first) {
-        if ((int)list.size() == first) return;
-        SnTask t;
-        t.front = -1; t.r0 = first; t.rows = (int)list.size() - first; t.c0 = 0; t.ncols = 0;
-        t.k = 0; t.nk = 1; t.chunk = -1; t.part = 0;
-        tasks.push_back(t);
-        first = (int)list.size();
-    };
-    // Bundles pay off where a level has many small fronts (throughput); on
-    // narrow levels a whole CTA per front keeps the dependency chain short.
-    std::vector<int> small_h(nsn + 1, 0), small_d(nsn + 1, 0);
-    for (int g = 0; g < nsn; ++g)
-        if (small_front(ncol[g] + nrow[g], ncol[g])) { ++small_h[height[g]]; ++small_d[depth[g]]; }
-    int bfirst = 0, blevel = -1;
-    for (int g : order) {
-        const int nj = ncol[g], m = nj + nrow[g];
-        if (height[g] != blevel) { flush(ftasks, bfwd, bfirst); blevel = height[g]; }
-        if (small_front(m, nj) && small_h[height[g]] >= kBundleLevel) {
-            bfwd.push_back(g);
-            ntf[g] = 1;
-            if ((int)bfwd.size() - bfirst == kWarps) flush(ftasks, bfwd, bfirst);
-            continue;
-        }
-        for (int r0 = 0; r0 < m; r0 += kRB) {
-            const int rowsb = std::min(kRB, m - r0);
-            const int cend = std::min(nj, r0 + kRB);
-            const int nk = std::max(1, (cend + kCC - 1) / kCC);
-            const int chunk = nk > 1 ? nchunk++ : -1;
-            const long long part = nk > 1 ? part_total : 0;
-            if (nk > 1) part_total += (long long)nk * kRB;
-            for (int k = 0; k < nk; ++k) {
-                SnTask t;
-                t.front = g; t.r0 = r0; t.rows = rowsb; t.c0 = k * kCC;
-                t.ncols = std::min(kCC, cend - k * kCC); t.k = k; t.nk = nk; t.chunk = chunk; t.part = part;
-                ftasks.push_back(t);
-                ++ntf[g];
-            }
-        }
-    }
-    flush(ftasks, bfwd, bfirst);
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return depth[a] < depth[b]; });
-    bfirst = 0;
-    blevel = -1;
-    for (int g : order) {
-        const int nj = ncol[g], m = nj + nrow[g];
-        if (depth[g] != blevel) { flush(btasks, bbwd, bfirst); blevel = depth[g]; }
-        if (small_front(m, nj) && small_d[depth[g]] >= kBundleLevel) {
-            bbwd.push_back(g);
-            ntb[g] = 1;
-            if ((int)bbwd.size() - bfirst == kWarps) flush(btasks, bbwd, bfirst);
-            continue;
-        }
-        // Column blocks of kBC columns over rows a0 .. m-1; a tall block is
-        // split into row chunks of kBRows (c0, ncols: the chunk's rows) whose
-        // partial sums the last chunk adds, so that the wide update part of a
-        // tall front is read by several CTAs at once.
-        for (int a0 = 0; a0 < nj; a0 += kBC) {
-            const int span = m - a0;
-            const int nk = std::max(1, (span + kBRows - 1) / kBRows);
-            const int chunk = nk > 1 ? nchunk++ : -1;
-            const long long part = nk > 1 ? part_total : 0;
-            if (nk > 1) part_total += (long long)nk * kBC;
-            for (int k = 0; k < nk; ++k) {
-                SnTask t;
-                t.front = g; t.r0 = a0; t.rows = std::min(kBC, nj - a0);
-                t.c0 = a0 + k * kBRows; t.ncols = std::min(kBRows, m - t.c0);
-                t.k = k; t.nk = nk; t.chunk = chunk; t.part = part;
-                btasks.push_back(t);
-                ++ntb[g];
-            }
-        }
-    }
-    flush(btasks, bbwd, bfirst);
-    // Algorithmic bytes: each stored coefficient of L_JJ^{-1} (lower triangle)
-    // and of -L_RJ L_JJ^{-1} read once per direction, plus b read and x written.
-    double coef = 0;
-    for (int g = 0; g < nsn; ++g) coef += 0.5 * ncol[g] * (ncol[g] + 1.0) + (double)nrow[g] * ncol[g];
-    fwd_bytes = 4.0 * coef + 8.0 * n;
-    bwd_bytes = 4.0 * coef + 8.0 * n;
-    n_fwd = (int)ftasks.size();
-    n_bwd = (int)btasks.size();
-    n_ctr = 2 + 2 * nsn + nchunk;
-    stamp("fronts and tasks");
-    // Coefficient blocks (FP64 -> FP32, padding rows zero), packed front by
-    // front into two pinned staging buffers in turn, each copied to the device
-    // while the next is packed: the gigabytes of a level-0 plan then cross at
-    // pinned-copy speed and the packing overlaps the copy.
-    size_t bytes_fw = 0;
-    {
-        const long long total = std::max<long long>(fw_total, 4);
-        d_fw = nullptr;
-        if (cudaMalloc(&d_fw, (size_t)total * sizeof(float)) != cudaSuccess)
-            throw Error(HDD_ERR_OUT_OF_MEMORY, "cudaMalloc: supernodal coefficients");
-        long long biggest = 4;
-        for (int g = 0; g < nsn; ++g) biggest = std::max(biggest, (long long)((ncol[g] + nrow[g] + 3) & ~3) * ncol[g]);
-        // Floats per staging buffer: 32 MB (pinning costs about as much as the
-        // copy, so the buffers stay small), or the largest front.
-        const long long chunk = std::max<long long>(biggest, 8ll << 20);
-        float* stage[2] = {nullptr, nullptr};
-        cudaEvent_t copied[2] = {nullptr, nullptr};
-        auto cleanup = [&]() {
-            for (int i = 0; i < 2; ++i) {
-                if (copied[i]) { cudaEventSynchronize(copied[i]); cudaEventDestroy(copied[i]); }
-                if (stage[i]) cudaFreeHost(stage[i]);
-            }
-        };
-        try {
-            for (int i = 0; i < 2; ++i) {
-                dev::ck(cudaMallocHost(&stage[i], (size_t)std::min(chunk, total) * sizeof(float)), "pinned staging");
-                dev::ck(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming), "event");
-            }
-            int g0 = 0, buf = 0;
-            bool used[2] = {false, false};
-            while (g0 < nsn) {
-                // Fronts g0 .. g1-1 fill this chunk (at least one front).
-                int g1 = g0 + 1;
-                while (g1 < nsn && fw_off[g1] + (long long)((ncol[g1] + nrow[g1] + 3) & ~3) * ncol[g1] -
-                                           fw_off[g0] <= chunk)
-                    ++g1;
-                const long long base = fw_off[g0];
-                const long long end = g1 < nsn ? fw_off[g1] : fw_total;
-                if (used[buf]) dev::ck(cudaEventSynchronize(copied[buf]), "staging reuse");
-                float* st = stage[buf];
-#pragma omp parallel for schedule(dynamic)
-                for (int g = g0; g < g1; ++g) {
-                    const SnFactor& F = *factors[where[g].first];
-                    const BlockVec& W = F.Fw[where[g].second];  // m x nj, col-major
-                    const int nj = ncol[g], m = nj + nrow[g], ld = (m + 3) & ~3;
-                    float* dst = st + (fw_off[g] - base);
-                    for (int c = 0; c < nj; ++c) {
-                        for (int r = 0; r < m; ++r) dst[(size_t)c * ld + r] = (float)W[(size_t)c * m + r];
-                        for (int r = m; r < ld; ++r) dst[(size_t)c * ld + r] = 0.0f;
-                    }
-                }
-                if (end > base)
-                    dev::ck(cudaMemcpyAsync(d_fw + base, st, (size_t)(end - base) * sizeof(float),
-                                            cudaMemcpyHostToDevice, s), "coefficient upload");
-                dev::ck(cudaEventRecord(copied[buf], s), "event");
-                used[buf] = true;
-                buf ^= 1;
-                g0 = g1;
-            }
-            if (fw_total < total)  // an empty plan's placeholder
-                dev::ck(cudaMemsetAsync(d_fw + fw_total, 0, (size_t)(total - fw_total) * sizeof(float), s), "memset");
-        } catch (...) {
-            cleanup();
-            throw;
-        }
-        cleanup();
-        bytes_fw = (size_t)total * sizeof(float);
-    }
-    stamp("coefficients packed and uploaded");
-    // Children lists and relative maps (child row -> position in parent's front).
-    relmap_off.assign(nsn, 0);
-    for (int g = 0; g < nsn; ++g) {
-        for (int c : kids[g]) child.push_back(c);
-        child_ptr.push_back((int)child.size());
-    }
-    {
-        long long total = 0;
-        for (int g = 0; g < nsn; ++g) {
-            relmap_off[g] = total;
-            if (parent_g[g] >= 0) total += nrow[g];
-        }
-        relmap.resize((size_t)total);
-        int bad = 0;
-#pragma omp parallel for schedule(dynamic, 64) reduction(| : bad)
-        for (int g = 0; g < nsn; ++g) {
-            const int p = parent_g[g];
-            if (p < 0) continue;
-            const int pc0 = col0[p], pnj = ncol[p];
-            const int* prow = rows.data() + rows_off[p];
-            const int pnr = nrow[p];
-            const int* crow = rows.data() + rows_off[g];
-            int* out = relmap.data() + relmap_off[g];
-            for (int kq = 0; kq < nrow[g]; ++kq) {
-                const int r = crow[kq];
-                int posn = 0;
-                if (r >= pc0 && r < pc0 + pnj) posn = r - pc0;
-                else {
-                    const int* it = std::lower_bound(prow, prow + pnr, r);
-                    if (it == prow + pnr || *it != r) bad = 1;
-                    else posn = pnj + (int)(it - prow);
-                }
-                out[kq] = posn;
-            }
-        }
-        if (bad) throw Error(HDD_ERR_INTERNAL, "supernode row not in parent front");
-    }
-    // Gather lists (the relative maps inverted per parent position, children
-    // in their order).
-    if (upd_total >= (long long)INT32_MAX) throw Error(HDD_ERR_UNSUPPORTED, "update vectors too large for 32-bit indices");
-    std::vector<long long> gp_off(nsn, 0), ge_off(nsn, 0);
-    std::vector<int> gptr, gent;
-    {
-        long long np = 0, ne = 0;
-        for (int g = 0; g < nsn; ++g) {
-            gp_off[g] = np;
-            ge_off[g] = ne;
-            np += ncol[g] + nrow[g] + 1;
-            for (int c = child_ptr[g]; c < child_ptr[g + 1]; ++c) ne += nrow[child[c]];
-        }
-        gptr.resize((size_t)np);
-        gent.resize((size_t)ne);
-#pragma omp parallel for schedule(dynamic, 64)
-        for (int g = 0; g < nsn; ++g) {
-            const int m = ncol[g] + nrow[g];
-            int* cnt = gptr.data() + gp_off[g];  // m + 1 entries
-            std::fill(cnt, cnt + m + 1, 0);
-            for (int c = child_ptr[g]; c < child_ptr[g + 1]; ++c) {
-                const int C = child[c];
-                for (int k = 0; k < nrow[C]; ++k) ++cnt[relmap[relmap_off[C] + k] + 1];
-            }
-            for (int q = 0; q < m; ++q) cnt[q + 1] += cnt[q];
-            std::vector<int> fill(cnt, cnt + m);
-            int* ent = gent.data() + ge_off[g];
-            for (int c = child_ptr[g]; c < child_ptr[g + 1]; ++c) {
-                const int C = child[c];
-                for (int k = 0; k < nrow[C]; ++k) {
-                    const int q = relmap[relmap_off[C] + k];
-                    ent[fill[q]++] = (int)(upd_off[C] + k);
-                }
-            }
-        }
-    }
-    stamp("relative maps and gather lists");
-    if (forward_smem(max_front, 1, nt) > 200 * 1024)
-        throw Error(HDD_ERR_UNSUPPORTED, "supernodal front too large for shared memory: " + std::to_string(max_front));
-    bytes = bytes_fw;
-    d_col0 = dev::upload(col0, s, bytes);
-    d_ncol = dev::upload(ncol, s, bytes);
-    d_nrow = dev::upload(nrow, s, bytes);
-    d_parent = dev::upload(parent_g, s, bytes);
-    d_rows = dev::upload(rows.empty() ? std::vector<int>{0} : rows, s, bytes);
-    d_rows_off = dev::upload(rows_off, s, bytes);
-    d_child_ptr = dev::upload(child_ptr, s, bytes);
-    d_child = dev::upload(child.empty() ? std::vector<int>{0} : child, s, bytes);
-    d_relmap_off = dev::upload(relmap_off, s, bytes);
-    d_gp_off = dev::upload(gp_off, s, bytes);
-    d_ge_off = dev::upload(ge_off, s, bytes);
-    d_gptr = dev::upload(gptr.empty() ? std::vector<int>{0} : gptr, s, bytes);
-    d_gent = dev::upload(gent.empty() ? std::vector<int>{0} : gent, s, bytes);
-    d_relmap = dev::upload(relmap.empty() ? std::vector<int>{0} : relmap, s, bytes);
-    d_upd_off = dev::upload(upd_off, s, bytes);
-    d_fw_off = dev::upload(fw_off, s, bytes);
-    d_ntf = dev::upload(ntf, s, bytes);
-    d_ntb = dev::upload(ntb, s, bytes);
-    d_perm = dev::upload(perm, s, bytes);
-    d_fwd = dev::upload(ftasks, s, bytes);
-    d_bwd = dev::upload(btasks, s, bytes);
-    d_bfwd = dev::upload(bfwd.empty() ? std::vector<int>{0} : bfwd, s, bytes);
-    d_bbwd = dev::upload(bbwd.empty() ? std::vector<int>{0} : bbwd, s, bytes);
-    stamp("uploads issued");
-    part_len = std::max<long long>(part_total, 1);
-    upd_len = std::max<long long>(upd_total, 1);
-    {
+    auto scratch = [&]() {
         PlanScratch sc;
         alloc_scratch(sc, shared_err, s, bytes);
         d_part = sc.part; d_upd = sc.upd; d_ynew = sc.ynew; d_xnew = sc.xnew; d_ctr = sc.ctr;
+        d_res = sc.res;
         d_err = sc.err;
         own_err = sc.own_err;
+    };
+    std::vector<int> base(factors.size() + 1, 0);
+    n = 0;
+    for (size_t f = 0; f < factors.size(); ++f) {
+        if (factors[f]->Fw.size() != factors[f]->col0.size()) throw Error(HDD_ERR_INTERNAL, "solve blocks not built");
+        n = std::max(n, offsets[f] + factors[f]->n);
+        base[f + 1] = base[f] + (int)factors[f]->col0.size();
     }
-    stamp("scratch allocated");
-    // A front with a parent, for stall_dependency (the wait of its parent's
-    // forward tasks on it can be made unsatisfiable).
+    nsn = base.back();
+    if (nsn == 0) return;
+    double total = 0;
+    for (const SnFactor* F : factors) total += tree_weight(*F);
+    if (shrink == 1 && resident_plan(factors, total) && res.build(factors, offsets, s)) {
+        kmax = 4;
+        solve_bytes = res.solve_bytes;
+        bytes = res.bytes;
+        scratch();
+        dev::ck(cudaStreamSynchronize(s), "plan upload");
+        stamp("resident plan uploaded");
+        return;
+    }
+    // The lower trees of every factor go to one CTA each (sn_resident.cu); the
+    // tasks below are those of the fronts above them.
+    std::vector<char> low(nsn, 0), cut_root(nsn, 0);
+    std::vector<ResidentPlan::Shape> shapes;
+    std::vector<int> shape_off;
+    std::vector<std::vector<int>> shape_roots;  // plan fronts of the trees' roots
+    const double cap = std::min(kCutMax, std::max(kCutMin, total / kCutShare)) / shrink;
+    for (size_t f = 0; f < factors.size(); ++f)
+        cut_trees(*factors[f], offsets[f], base[f], cap, low, cut_root, shapes, shape_off, shape_roots);
+    // The fronts above, numbered in post-order, factor by factor.  Members given
+    // the same factor share its coefficients.
+    struct Front {
+        int f, j, nj, nr, col0, parent, height, depth, upd;
+        long long fw, rows_off, gp, ge;
+        std::vector<int> kids;  // plan fronts (trees' roots among them), in order
+        int child_b, child_e, ntf, ntb;
+    };
+    std::vector<Front> top;
+    std::vector<int> top_of(nsn, -1);
+    std::vector<int> upd_off(nsn, -1);  // of the fronts above and the trees' roots
+    std::vector<int> own;               // fronts whose coefficients are stored
+    std::map<const SnFactor*, size_t> first_of;
+    long long upd_total = 0, fw_total = 0;
+    max_front = 0;
+    std::vector<int> rows, perm(n, 0);
+    for (size_t f = 0; f < factors.size(); ++f) {
+        const SnFactor& F = *factors[f];
+        const size_t owner = first_of.emplace(&F, f).first->second;
+        for (int i = 0; i < F.n; ++i) perm[offsets[f] + i] = offsets[f] + F.perm[i];
+        for (int j = 0; j < (int)F.col0.size(); ++j) {
+            const int g = base[f] + j, nr = (int)F.rows[j].size();
+            if (!low[g] || cut_root[g]) {
+                if (upd_total + nr >= (long long)INT32_MAX)
+                    throw Error(HDD_ERR_UNSUPPORTED, "update vectors too large for 32-bit indices");
+                upd_off[g] = (int)upd_total;
+                upd_total += nr;
+            }
+            if (low[g]) continue;
+            Front T{};
+            T.f = (int)f; T.j = j; T.nj = F.ncol[j]; T.nr = nr; T.col0 = offsets[f] + F.col0[j]; T.upd = upd_off[g];
+            T.rows_off = (long long)rows.size();
+            for (int r : F.rows[j]) rows.push_back(offsets[f] + r);
+            const long long len = (long long)((T.nj + nr + 3) & ~3) * T.nj;
+            if (owner == f) {
+                own.push_back((int)top.size());
+                T.fw = fw_total;
+                fw_total += len;
+            } else {
+                T.fw = top[top_of[base[owner] + j]].fw;
+            }
+            max_front = std::max(max_front, T.nj + nr);
+            top_of[g] = (int)top.size();
+            top.push_back(std::move(T));
+        }
+        for (int j = 0; j < (int)F.col0.size(); ++j) {
+            const int p = F.parent[j], g = base[f] + j;
+            if (top_of[g] >= 0) top[top_of[g]].parent = p >= 0 ? top_of[base[f] + p] : -1;
+            if (p >= 0 && top_of[base[f] + p] >= 0) top[top_of[base[f] + p]].kids.push_back(g);
+        }
+    }
+    for (size_t i = 0; i < shapes.size(); ++i)
+        for (size_t t = 0; t < shapes[i].trees.size(); ++t) {
+            ResidentPlan::Tree& tree = shapes[i].trees[t];
+            if (!shapes[i].F->rows[tree.last].empty()) tree.top = upd_off[shape_roots[i][t]];
+        }
+    if (!shapes.empty() && !res.build_cut(shapes, shape_off, s)) {
+        // Trees with unusually many update entries: smaller ones, in the end none.
+        build(factors, offsets, s, shared_err, shrink * 4);
+        return;
+    }
+    stamp("trees uploaded");
+    ntop = (int)top.size();
+    for (int t = 0; t < ntop; ++t)
+        if (top[t].parent >= 0) top[top[t].parent].height = std::max(top[top[t].parent].height, top[t].height + 1);
+    for (int t = ntop - 1; t >= 0; --t)
+        if (top[t].parent >= 0) top[t].depth = top[top[t].parent].depth + 1;
+    // Tasks in topological order.
+    std::vector<int> order(ntop);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return top[a].height < top[b].height; });
+    std::vector<SnTask> tasks;
+    int nchunk = 0;
+    long long part_total = 0;
+    auto task_of = [&](int t) {
+        const Front& T = top[t];
+        SnTask k{};
+        k.front = t; k.nj = T.nj; k.m = T.nj + T.nr; k.col0 = T.col0; k.upd = T.upd; k.parent = T.parent;
+        k.rows_off = T.rows_off;
+        return k;
+    };
+    for (int t : order) {
+        const int nj = top[t].nj, m = nj + top[t].nr;
+        for (int r0 = 0; r0 < m; r0 += kRB) {
+            const int cend = std::min(nj, r0 + kRB);
+            const int nk = cend <= kWhole ? 1 : (cend + kCC - 1) / kCC;
+            SnTask k = task_of(t);
+            k.r0 = r0; k.rows = std::min(kRB, m - r0); k.nk = nk;
+            k.chunk = nk > 1 ? nchunk++ : -1;
+            k.part = part_total;
+            if (nk > 1) part_total += (long long)nk * kRB;
+            for (k.k = 0; k.k < nk; ++k.k) {
+                k.c0 = k.k * kCC;
+                k.ncols = nk > 1 ? std::min(kCC, cend - k.c0) : cend;
+                tasks.push_back(k);
+                ++top[t].ntf;
+            }
+        }
+    }
+    n_fwd = (int)tasks.size();
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return top[a].depth < top[b].depth; });
+    for (int t : order) {
+        const int nj = top[t].nj, m = nj + top[t].nr;
+        const int cw = m <= kTallRows ? 4 : 2, bc = cols_of(cw), br = rows_of(cw);
+        for (int a0 = 0; a0 < nj; a0 += bc) {
+            const int nk = (m - a0 + br - 1) / br;
+            SnTask k = task_of(t);
+            k.r0 = a0; k.rows = std::min(bc, nj - a0); k.nk = nk; k.cw = cw;
+            k.chunk = nk > 1 ? nchunk++ : -1;
+            k.part = part_total;
+            if (nk > 1) part_total += (long long)nk * bc;
+            for (k.k = 0; k.k < nk; ++k.k) {
+                k.c0 = a0 + k.k * br;
+                k.ncols = std::min(br, m - k.c0);
+                tasks.push_back(k);
+                ++top[t].ntb;
+            }
+        }
+    }
+    n_tasks = (int)tasks.size();
+    ld_ctr = 2 * ntop + nchunk;
+    // Algorithmic bytes: each stored coefficient of L_JJ^{-1} (lower triangle)
+    // and of -L_RJ L_JJ^{-1} read once per direction, plus b read and x written.
+    double coef = 0;
+    for (int t : own) coef += 0.5 * top[t].nj * (top[t].nj + 1.0) + (double)top[t].nr * top[t].nj;
+    solve_bytes = 8.0 * coef + 8.0 * n + res.solve_bytes;
+    stamp("fronts and tasks");
+    // Coefficient blocks (FP64 -> FP32, padding rows zero) of the distinct
+    // factors' fronts.
+    bytes = res.bytes;
+    dev::upload_packed(own.size(), fw_total, [&](size_t i) { return top[own[i]].fw; },
+                       [&](size_t i, float* dst) {
+                           const Front& T = top[own[i]];
+                           const BlockVec& W = factors[T.f]->Fw[T.j];  // m x nj, col-major
+                           const int m = T.nj + T.nr, ld = (m + 3) & ~3;
+                           for (int c = 0; c < T.nj; ++c) {
+                               for (int r = 0; r < m; ++r) dst[(size_t)c * ld + r] = (float)W[(size_t)c * m + r];
+                               for (int r = m; r < ld; ++r) dst[(size_t)c * ld + r] = 0.0f;
+                           }
+                       },
+                       s, d_fw, bytes);
+    stamp("coefficients packed and uploaded");
+    // Gather lists: the children's update entries per position of a front, in
+    // child order; and the children it waits for.
+    std::vector<int> child, gptr, gent;
+    {
+        long long np = 0, ne = 0;
+        for (Front& T : top) {
+            T.gp = np;
+            T.ge = ne;
+            np += T.nj + T.nr + 1;
+            T.child_b = (int)child.size();
+            for (int g : T.kids) {
+                const size_t f = (size_t)T.f;
+                ne += (long long)factors[f]->rows[g - base[f]].size();
+                if (top_of[g] >= 0) child.push_back(top_of[g]);
+            }
+            T.child_e = (int)child.size();
+        }
+        gptr.resize((size_t)np);
+        gent.resize((size_t)ne);
+        int bad = 0;
+#pragma omp parallel for schedule(dynamic, 8) reduction(| : bad)
+        for (int t = 0; t < ntop; ++t) {
+            const Front& T = top[t];
+            const SnFactor& F = *factors[T.f];
+            const int m = T.nj + T.nr, c0 = F.col0[T.j];
+            const std::vector<int>& R = F.rows[T.j];
+            int* cnt = gptr.data() + T.gp;  // m + 1 entries
+            std::fill(cnt, cnt + m + 1, 0);
+            std::vector<int> pos;  // position of every child entry, child by child
+            for (int g : T.kids)
+                for (int r : F.rows[g - base[T.f]]) {
+                    int p = 0;
+                    if (r >= c0 && r < c0 + T.nj) p = r - c0;
+                    else {
+                        const auto it = std::lower_bound(R.begin(), R.end(), r);
+                        if (it == R.end() || *it != r) bad = 1;
+                        else p = T.nj + (int)(it - R.begin());
+                    }
+                    pos.push_back(p);
+                    ++cnt[p + 1];
+                }
+            for (int q = 0; q < m; ++q) cnt[q + 1] += cnt[q];
+            std::vector<int> fill(cnt, cnt + m);
+            int* ent = gent.data() + T.ge;
+            size_t i = 0;
+            for (int g : T.kids)
+                for (size_t k = 0; k < F.rows[g - base[T.f]].size(); ++k) ent[fill[pos[i++]]++] = upd_off[g] + (int)k;
+        }
+        if (bad) throw Error(HDD_ERR_INTERNAL, "supernode row not in parent front");
+    }
+    for (SnTask& k : tasks) {
+        const Front& T = top[k.front];
+        k.fw = T.fw;
+        k.gp = T.gp;
+        k.ge = T.ge;
+        k.child_b = T.child_b;
+        k.child_e = T.child_e;
+        k.kids = T.kids.empty() ? 0 : 1;
+    }
+    stamp("gather lists");
+    if (front_bytes(max_front, 1) > kFrontMax)
+        throw Error(HDD_ERR_UNSUPPORTED, "supernodal front too large: " + std::to_string(max_front));
+    kmax = 1;
+    for (int k : {2, 4})
+        if (front_bytes(max_front, k) <= kSmemMax) kmax = k;
+    std::vector<int> ntf, ntb;
+    for (const Front& T : top) {
+        ntf.push_back(T.ntf);
+        ntb.push_back(T.ntb);
+    }
+    auto nonempty = [](std::vector<int>& v) -> const std::vector<int>& {
+        if (v.empty()) v.push_back(0);
+        return v;
+    };
+    d_rows = dev::upload(nonempty(rows), s, bytes);
+    d_child = dev::upload(nonempty(child), s, bytes);
+    d_gptr = dev::upload(nonempty(gptr), s, bytes);
+    d_gent = dev::upload(nonempty(gent), s, bytes);
+    d_ntf = dev::upload(nonempty(ntf), s, bytes);
+    d_ntb = dev::upload(nonempty(ntb), s, bytes);
+    d_perm = dev::upload(perm, s, bytes);
+    if (tasks.empty()) tasks.push_back(SnTask{});
+    d_tasks = dev::upload(tasks, s, bytes);
+    stamp("uploads issued");
+    part_len = std::max<long long>(part_total, 1);
+    upd_len = std::max<long long>(upd_total, 1);
+    scratch();
+    // A front with a child above the trees, for stall_dependency (the wait of its
+    // tasks on that child can be made unsatisfiable).
     stall_front = -1;
-    stall_ntf = 0;
-    for (int g = 0; g < nsn; ++g)
-        if (parent_g[g] >= 0) { stall_front = g; stall_ntf = ntf[g]; break; }
-    ntasks_f = n_fwd;
-    ntasks_b = n_bwd;
-    // Persistent grid: as many CTAs as fit on the device, per right-hand-side
-    // count whose shared memory fits; no more than tasks at launch.
-    int dev_id = 0, nsm = 0;
+    for (int t = 0; t < ntop && stall_front < 0; ++t)
+        if (top[t].parent >= 0) { stall_front = t; stall_ntf = top[t].ntf; }
+    // Persistent grid: as many CTAs as fit on the device; no more than tasks.
+    int dev_id = 0, nsm = 0, per_sm = 0;
     dev::ck(cudaGetDevice(&dev_id), "cudaGetDevice");
     dev::ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev_id), "SM count");
-    kmax = 1;
-    for (int i = 0; i < 3; ++i) {
-        const int k = kBatches[i];
-        const size_t smf = forward_smem(max_front, k, nt), smb = backward_smem(max_front, k, nt);
-        grids[i] = 0;
-        if (std::max(smf, smb) > kSmemMax) break;
-        raise_smem_limit(dev_id, k, nt, (int)std::max(smf, smb));
-        const int occ = nt == kNTInterior ? occupancy_nt<kNTInterior>(k, smf, smb) : occupancy_nt<kNTInterface>(k, smf, smb);
-        grids[i] = std::max(1, nsm * occ);
-        kmax = k;
-    }
-    grid = grids[0];
-    stamp("grids sized");
+    dev::ck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sn_task_kernel, kNT, 0), "occupancy");
+    grid = std::max(1, nsm * std::max(1, per_sm));
     dev::ck(cudaStreamSynchronize(s), "plan upload");
     stamp("uploaded");
 }
 
 void SolvePlan::release() {
-    dev::release(d_col0); dev::release(d_ncol); dev::release(d_nrow); dev::release(d_parent);
-    dev::release(d_rows); dev::release(d_rows_off); dev::release(d_child_ptr); dev::release(d_child);
-    dev::release(d_relmap_off); dev::release(d_relmap);
-    dev::release(d_gp_off); dev::release(d_ge_off); dev::release(d_gptr); dev::release(d_gent); dev::release(d_upd_off); dev::release(d_fw_off);
-    dev::release(d_ntf); dev::release(d_ntb); dev::release(d_perm);
-    dev::release(d_fwd); dev::release(d_bwd); dev::release(d_bfwd); dev::release(d_bbwd); dev::release(d_fw); dev::release(d_part); dev::release(d_upd);
-    dev::release(d_ynew); dev::release(d_xnew); dev::release(d_ctr);
+    dev::release(d_rows); dev::release(d_child); dev::release(d_gptr); dev::release(d_gent);
+    dev::release(d_ntf); dev::release(d_ntb); dev::release(d_perm); dev::release(d_tasks); dev::release(d_fw);
+    dev::release(d_part); dev::release(d_upd); dev::release(d_ynew); dev::release(d_xnew); dev::release(d_ctr);
+    dev::release(d_res.upd); dev::release(d_res.y);
     if (own_err) dev::release(d_err);
+    res.release();
     d_err = nullptr;
     own_err = false;
-    nsn = 0;
-    n = 0;
-    n_fwd = n_bwd = n_ctr = 0;
+    nsn = ntop = n = n_fwd = n_tasks = ld_ctr = 0;
+    part_len = upd_len = 0;
+    stall_front = -1;
+    bytes = 0;
 }
 
 void SolvePlan::alloc_scratch(PlanScratch& sc, int* shared_err, cudaStream_t s, size_t& b, int nrhs) const {
     if (nrhs != 1 && nrhs != 2 && nrhs != 4) throw Error(HDD_ERR_INVALID_ARGUMENT, "right-hand sides per solve: 1, 2 or 4");
     sc.nrhs = nrhs;
-    sc.part = dev::alloc_zero<double>(part_len * nrhs, b, s);
-    sc.upd = dev::alloc_zero<double>(upd_len * nrhs, b, s);
-    sc.ynew = dev::alloc_zero<double>((long long)std::max(n, 1) * nrhs, b, s);
-    sc.xnew = dev::alloc_zero<double>((long long)std::max(n, 1) * nrhs, b, s);
-    sc.ctr = dev::alloc_zero<int>(std::max(n_ctr, 1), b, s);
+    if (res.ngroups > 0) {
+        sc.res.upd = dev::alloc_zero<double>(res.upd_len * nrhs, b, s);
+        sc.res.y = dev::alloc_zero<double>(res.y_len * nrhs, b, s);
+    }
+    if (!whole_resident()) {
+        sc.part = dev::alloc_zero<double>(part_len * nrhs, b, s);
+        sc.upd = dev::alloc_zero<double>(upd_len * nrhs, b, s);
+        sc.ynew = dev::alloc_zero<double>((long long)std::max(n, 1) * nrhs, b, s);
+        sc.xnew = dev::alloc_zero<double>((long long)std::max(n, 1) * nrhs, b, s);
+        sc.ctr = dev::alloc_zero<int>(1 + (size_t)ld_ctr * nrhs, b, s);
+    }
     if (shared_err) {
         sc.err = shared_err;
         sc.own_err = false;
@@ -1108,8 +847,17 @@ void SolvePlan::alloc_scratch(PlanScratch& sc, int* shared_err, cudaStream_t s, 
     }
 }
 
+size_t SolvePlan::scratch_bytes(int nrhs) const {
+    if (nsn == 0) return 0;
+    size_t t = 4 + (size_t)nrhs * 8 * (size_t)(res.upd_len + res.y_len);
+    if (!whole_resident())
+        t += (size_t)nrhs * (8 * (size_t)(part_len + upd_len) + 16 * (size_t)std::max(n, 1) + 4 * (size_t)ld_ctr) + 4;
+    return t;
+}
+
 void SolvePlan::free_scratch(PlanScratch& sc) {
     dev::release(sc.part); dev::release(sc.upd); dev::release(sc.ynew); dev::release(sc.xnew); dev::release(sc.ctr);
+    dev::release(sc.res.upd); dev::release(sc.res.y);
     if (sc.own_err) dev::release(sc.err);
     sc.err = nullptr;
     sc.own_err = false;
@@ -1118,6 +866,7 @@ void SolvePlan::free_scratch(PlanScratch& sc) {
 PlanScratch SolvePlan::primary() const {
     PlanScratch sc;
     sc.part = d_part; sc.upd = d_upd; sc.ynew = d_ynew; sc.xnew = d_xnew; sc.ctr = d_ctr; sc.err = d_err;
+    sc.res = d_res;
     sc.own_err = false;
     sc.nrhs = 1;
     return sc;
@@ -1127,50 +876,44 @@ void SolvePlan::solve(const float* b_old, float* x_old, cudaStream_t s, long lon
     solve(primary(), b_old, x_old, s, launches, hook);
 }
 
-template <int K, int NT>
-static void launch_pair(const PlanView& P, int g, int n_fwd, int n_bwd, int max_front, const SnTask* fwd,
-                        const SnTask* bwd, const float* b_old, float* x_old, cudaStream_t s, PhaseHook* hook,
-                        double fwd_bytes, double bwd_bytes) {
-    if (hook) hook->begin(kPhaseSnForward);
-    sn_forward_kernel<K, NT><<<std::min(g, n_fwd), NT, forward_smem(max_front, K, NT), s>>>(P, fwd, n_fwd, b_old);
-    dev::ck(cudaGetLastError(), "sn forward");
-    if (hook) hook->end(kPhaseSnForward, fwd_bytes);
-    if (hook) hook->begin(kPhaseSnBackward);
-    sn_backward_kernel<K, NT><<<std::min(g, n_bwd), NT, backward_smem(max_front, K, NT), s>>>(P, bwd, n_bwd,
-                                                                                          x_old);
-    dev::ck(cudaGetLastError(), "sn backward");
-    if (hook) hook->end(kPhaseSnBackward, bwd_bytes);
-}
-
 void SolvePlan::solve(const PlanScratch& sc, const float* b_old, float* x_old, cudaStream_t s, long long& launches,
                       PhaseHook* hook, int nrhs, long long ld_b, long long ld_x) const {
     if (nsn == 0) return;
     if ((nrhs != 1 && nrhs != 2 && nrhs != 4) || nrhs > sc.nrhs || nrhs > kmax)
         throw Error(HDD_ERR_INVALID_ARGUMENT, "right-hand sides per solve: 1, 2 or 4, within the scratch and the plan");
-    PlanView P{nsn, max_front, d_col0, d_ncol, d_nrow, d_parent, d_rows, d_rows_off, d_child_ptr, d_child,
-               d_relmap_off, d_relmap, d_gp_off, d_ge_off, d_gptr, d_gent, d_upd_off, d_fw_off, d_ntf, d_ntb, d_perm,
-               d_bfwd, d_bbwd, d_fw, sc.part, sc.upd,
-               sc.ynew, sc.xnew, sc.ctr, sc.err, spin_limit,
-               part_len, upd_len, (long long)std::max(n, 1), ld_b, ld_x};
-    dev::ck(cudaMemsetAsync(sc.ctr, 0, sizeof(int) * n_ctr, s), "reset counters");
-    const int slot = nrhs == 1 ? 0 : (nrhs == 2 ? 1 : 2);
-    const int full = grids[slot];
-    const int g = sc.grid_div > 1 ? std::max(1, (full + sc.grid_div - 1) / sc.grid_div) : full;
-    const double fb = fwd_bytes + 8.0 * n * (nrhs - 1), bb = bwd_bytes + 8.0 * n * (nrhs - 1);
-    if (nt == kNTInterior) {
-        if (nrhs == 1) launch_pair<1, kNTInterior>(P, g, n_fwd, n_bwd, max_front, d_fwd, d_bwd, b_old, x_old, s, hook, fb, bb);
-        else if (nrhs == 2) launch_pair<2, kNTInterior>(P, g, n_fwd, n_bwd, max_front, d_fwd, d_bwd, b_old, x_old, s, hook, fb, bb);
-        else launch_pair<4, kNTInterior>(P, g, n_fwd, n_bwd, max_front, d_fwd, d_bwd, b_old, x_old, s, hook, fb, bb);
+    if (hook) hook->begin(kPhaseSolve);
+    const TopVectors top{sc.upd, sc.xnew, upd_len, (long long)std::max(n, 1), sc.ctr,
+                         sc.ctr ? 1 + (long long)ld_ctr * nrhs : 0};
+    auto trees = [&](int mode) {
+        res.launch(mode, sc.res, top, sc.err, sc.grid_div, spin_limit, b_old, x_old, s, nrhs, ld_b, ld_x);
+        ++launches;
+    };
+    if (whole_resident()) {
+        trees(0);
     } else {
-        if (nrhs == 1) launch_pair<1, kNTInterface>(P, g, n_fwd, n_bwd, max_front, d_fwd, d_bwd, b_old, x_old, s, hook, fb, bb);
-        else if (nrhs == 2) launch_pair<2, kNTInterface>(P, g, n_fwd, n_bwd, max_front, d_fwd, d_bwd, b_old, x_old, s, hook, fb, bb);
-        else launch_pair<4, kNTInterface>(P, g, n_fwd, n_bwd, max_front, d_fwd, d_bwd, b_old, x_old, s, hook, fb, bb);
+        // The forward launch of the trees clears the counters.
+        if (res.ngroups > 0) trees(1);
+        else dev::ck(cudaMemsetAsync(sc.ctr, 0, sizeof(int) * (size_t)top.n_ctr, s), "reset counters");
+        if (n_tasks > 0) {
+            const PlanView P{ntop, n_fwd, n_tasks, d_rows, d_child, d_gptr, d_gent, d_ntf, d_ntb, d_perm, d_fw,
+                             d_tasks, b_old, x_old, sc.part, sc.upd, sc.ynew, sc.xnew, sc.ctr, sc.err, spin_limit,
+                             part_len, upd_len, (long long)std::max(n, 1), ld_ctr, ld_b, ld_x, nrhs};
+            const int full = std::min(grid, n_tasks * nrhs);
+            const int g = sc.grid_div > 1 ? std::min(full, std::max(1, (grid + sc.grid_div - 1) / sc.grid_div)) : full;
+            sn_task_kernel<<<g, kNT, 0, s>>>(P);
+            dev::ck(cudaGetLastError(), "sn tasks");
+            ++launches;
+        }
+        if (res.ngroups > 0) trees(2);
     }
-    launches += 2;
+    if (hook) hook->end(kPhaseSolve, solve_bytes + 16.0 * n * (nrhs - 1));
 }
 
 void SolvePlan::stall_dependency(bool on, cudaStream_t s) {
-    if (stall_front < 0) return;
+    if (stall_front < 0) {
+        if (res.ngroups > 0) res.set_gate(on ? 1 : 0, s);
+        return;
+    }
     const int v = on ? stall_ntf + 1 : stall_ntf;
     dev::ck(cudaMemcpyAsync(d_ntf + stall_front, &v, sizeof(int), cudaMemcpyHostToDevice, s), "stall dependency");
     dev::ck(cudaStreamSynchronize(s), "stall dependency");

@@ -272,7 +272,7 @@ struct Solver {
     void sigma_vcycle_host(const float* b0, float* u0);
     // One Arr (kind 0) or concatenated Aii (kind 1) supernodal solve of a sigma level.
     void interface_solve(int kind, int level, const float* bh, float* xh, int* n);
-    // The same for nrhs (1, 2 or 4) right-hand sides solved in one launch pair.
+    // The same for nrhs (1, 2 or 4) right-hand sides solved by the same launches.
     void interface_solve_batch(int kind, int level, int nrhs, const float* bh, float* xh, int* n);
     // Throws HDD_ERR_TIMEOUT when a device-side bounded wait gave up.
     void check_waits() { check_waits(w0); }

@@ -252,9 +252,9 @@ hdd_status hdd_sigma_vcycle(hdd_solver* s, const float* b0, float* u0);
 hdd_status hdd_interface_solve(hdd_solver* s, int kind, int level, const float* b, float* x, int* n);
 
 /* Test seam: the same for nrhs (1, 2 or 4) right-hand sides at once, b and x
- * holding nrhs vectors of *n entries one after another.  One launch pair
- * reads each coefficient once for all of them; each solution is bit-identical
- * to hdd_interface_solve of its right-hand side.  HDD_ERR_UNSUPPORTED when the
+ * holding nrhs vectors of *n entries one after another.  The same
+ * launches take all of them; each solution is bit-identical to
+ * hdd_interface_solve of its right-hand side.  HDD_ERR_UNSUPPORTED when the
  * plan's largest front leaves no shared memory for nrhs vectors. */
 hdd_status hdd_interface_solve_batch(hdd_solver* s, int kind, int level, int nrhs, const float* b, float* x, int* n);
 
@@ -271,11 +271,11 @@ hdd_status hdd_interface_matrix(hdd_solver* s, int kind, int level, int subdomai
 /* Per-phase device timing (CUDA events on the solver stream) for profiling;
  * no reference counterpart (the reference prints wall-clock times).
  * Phases: 0 V-cycle kernel, 1 Laplacian kernel, 2 PCG vector kernels,
- * 3 interface gather/scatter, 4 sigma V-cycle (includes 6 and 7), 5 dense<->
- * tile copies, 6 supernodal forward solves, 7 supernodal backward solves.
+ * 3 interface gather/scatter, 4 sigma V-cycle (includes 6), 5 dense<->
+ * tile copies, 6 supernodal solves (forward and backward), 7 none.
  * Enabling clears the accumulators; ms/launches/bytes hold 8 entries.
  * hdd_get_kernel_bytes gives each phase's algorithmic bytes (the data the
- * kernels must move at minimum) for phases 0, 1, 6 and 7, 0 for the others. */
+ * kernels must move at minimum) for phases 0, 1 and 6, 0 for the others. */
 hdd_status hdd_set_kernel_timing(hdd_solver* s, int enable);
 hdd_status hdd_get_kernel_timing(hdd_solver* s, double* ms, long long* launches);
 hdd_status hdd_get_kernel_bytes(hdd_solver* s, double* bytes);

@@ -269,6 +269,12 @@ int shim_matrix_get(void* h, int kind, int level, int sub, int* ptr, int* col, d
     return 0;
 }
 
+// rep[i]: the first subdomain whose interior system of the level equals i's.
+void shim_interior_classes(void* h, int level, int* rep) {
+    const std::vector<int> r = interior_classes(static_cast<Shim*>(h)->ih, level);
+    for (size_t i = 0; i < r.size(); ++i) rep[i] = r[i];
+}
+
 // Factor (A + 1e-5 I) of one matrix with the supernodal Cholesky (geometric
 // ordering when positions exist), solve for a random right-hand side on the
 // host and return ||(A + 1e-5 I) x - b|| / ||b||; also checks that the explicit

@@ -51,6 +51,7 @@ def load_shim():
     L.shim_setup_digest.argtypes = [C.c_void_p]
     L.shim_factor_components.restype = C.c_double
     L.shim_factor_components.argtypes = [C.c_int, C.c_int]
+    L.shim_interior_classes.argtypes = [C.c_void_p, C.c_int, ip]
     L.shim_factor_check.restype = C.c_double
     L.shim_factor_check.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double)]
     L.shim_plan_check.restype = C.c_double
