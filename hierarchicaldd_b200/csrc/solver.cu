@@ -330,7 +330,7 @@ void Solver::initialize() {
 
 void Solver::alloc_vectors(Work& w) {
     const size_t nt = L.tiles.size(), N = std::max<size_t>(nt * (size_t)L.tile_cells, 1);
-    const size_t P = std::max<size_t>({nt, (size_t)laplace_partials(geom()), (size_t)1});
+    const size_t P = std::max<size_t>({(size_t)vector_partials(geom()), (size_t)laplace_partials(geom()), (size_t)1});
     const size_t k = (size_t)w.k;
     w.vstride = N;
     w.pstride = (int)P;
@@ -389,7 +389,7 @@ std::unique_ptr<Work> Solver::make_work(int k) {
 
 size_t Solver::work_bytes(int k) const {
     const size_t nt = L.tiles.size(), N = nt * (size_t)L.tile_cells;
-    const size_t P = std::max<size_t>({nt, (size_t)laplace_partials(geom()), (size_t)1});
+    const size_t P = std::max<size_t>({(size_t)vector_partials(geom()), (size_t)laplace_partials(geom()), (size_t)1});
     size_t t = std::max<size_t>(L.cell_count(), 1) * 4 + (opts.multilevel ? 7 : 6) * std::max<size_t>(N, 1) * 4 * k;
     if (opts.precision_mode == HDD_PRECISION_MIXED) t += std::max<size_t>(N, 1) * 8 * k;
     t += (P * 12 + 128 + sizeof(PcgScalars) + 12) * k;
@@ -693,7 +693,7 @@ void Solver::solve(Work& w, hdd_result* res) {
     NvtxRange range("solve");
     cuda_check(cudaSetDevice(opts.device), "cudaSetDevice");
     const TileGeom g = geom();
-    const int nt = g.ntiles;
+    const int nv = vector_partials(g);
     const int mode = opts.precision_mode == HDD_PRECISION_MIXED ? 1 : 0;
     PcgScalars init;
     std::memset(&init, 0, sizeof(init));
@@ -710,7 +710,7 @@ void Solver::solve(Work& w, hdd_result* res) {
     cuda_check(cudaEventRecord(e0, w.stream), "event record");
     // r = Project(b - A x) with x = 0 (restart branch, CONJUGATE_GRADIENT.cpp:36).
     cuda_check(launch_residual(g, w.b.p, w.x.p, w.r.p, w.partial_max.p, w.stream), "residual"); count(w);
-    cuda_check(launch_reduce_max(w.partial_max.p, nt, w.scalars_f.p, w.stream), "reduce"); count(w);
+    cuda_check(launch_reduce_max(w.partial_max.p, nv, w.scalars_f.p, w.stream), "reduce"); count(w);
     float rmax = 0;
     PcgScalars hs;
     cuda_check(cudaMemcpyAsync(&rmax, w.scalars_f.p, sizeof(float), cudaMemcpyDeviceToHost, w.stream), "D2H");
@@ -739,7 +739,7 @@ void Solver::solve(Work& w, hdd_result* res) {
         if (rmax <= threshold && (it >= opts.min_iters || rmax < small_number)) {
             if (mode != 1 || replaced) { converged = true; break; }
             cuda_check(launch_residual_f64(g, w.b.p, xdp, w.r.p, w.partial_max.p, w.stream), "true residual"); count(w);
-            cuda_check(launch_reduce_max(w.partial_max.p, nt, w.scalars_f.p, w.stream), "reduce"); count(w);
+            cuda_check(launch_reduce_max(w.partial_max.p, nv, w.scalars_f.p, w.stream), "reduce"); count(w);
             cuda_check(cudaMemcpyAsync(&rmax, w.scalars_f.p, sizeof(float), cudaMemcpyDeviceToHost, w.stream), "D2H");
             sync(w);
             w.history.back() = (double)rmax;
@@ -755,7 +755,7 @@ void Solver::solve(Work& w, hdd_result* res) {
         {
             Tm tm(this, w, 2);
             cuda_check(launch_project_dot(g, w.z.p, w.r.p, w.partial.p, w.stream), "project_dot"); count(w);
-            cuda_check(launch_reduce_sum(w.partial.p, nt, w.sums.p + 0, w.stream), "reduce"); count(w);
+            cuda_check(launch_reduce_sum(w.partial.p, nv, w.sums.p + 0, w.stream), "reduce"); count(w);
             cuda_check(launch_scalar_rho(w.scal.p, w.sums.p + 0, first, w.stream), "rho"); count(w);
             cuda_check(launch_update_s(g, w.s.p, w.z.p, w.scal.p, first, mode, w.stream), "update_s"); count(w);
         }
@@ -774,7 +774,7 @@ void Solver::solve(Work& w, hdd_result* res) {
             cuda_check(launch_residual_f64(g, w.b.p, xdp, w.r.p, w.partial_max.p, w.stream), "true residual"); count(w);
             replaced = true;
         }
-        cuda_check(launch_reduce_max(w.partial_max.p, nt, w.scalars_f.p, w.stream), "reduce"); count(w);
+        cuda_check(launch_reduce_max(w.partial_max.p, nv, w.scalars_f.p, w.stream), "reduce"); count(w);
         cuda_check(cudaMemcpyAsync(&rmax, w.scalars_f.p, sizeof(float), cudaMemcpyDeviceToHost, w.stream), "D2H");
         cuda_check(cudaMemcpyAsync(&hs, w.scal.p, sizeof(hs), cudaMemcpyDeviceToHost, w.stream), "D2H");
         int herr = 0, herr2 = 0;
@@ -803,11 +803,11 @@ void Solver::solve(Work& w, hdd_result* res) {
     if (xdp) cuda_check(launch_residual_f64(g, w.b.p, xdp, w.q.p, w.partial_max.p, w.stream), "true residual");
     else cuda_check(launch_residual(g, w.b.p, w.x.p, w.q.p, w.partial_max.p, w.stream), "true residual");
     count(w);
-    cuda_check(launch_reduce_max(w.partial_max.p, nt, w.scalars_f.p + 1, w.stream), "reduce"); count(w);
+    cuda_check(launch_reduce_max(w.partial_max.p, nv, w.scalars_f.p + 1, w.stream), "reduce"); count(w);
     cuda_check(launch_project_dot(g, w.q.p, w.q.p, w.partial.p, w.stream), "dot"); count(w);
-    cuda_check(launch_reduce_sum(w.partial.p, nt, w.sums.p + 2, w.stream), "reduce"); count(w);
+    cuda_check(launch_reduce_sum(w.partial.p, nv, w.sums.p + 2, w.stream), "reduce"); count(w);
     cuda_check(launch_project_dot(g, w.b.p, w.b.p, w.partial.p, w.stream), "dot"); count(w);
-    cuda_check(launch_reduce_sum(w.partial.p, nt, w.sums.p + 3, w.stream), "reduce"); count(w);
+    cuda_check(launch_reduce_sum(w.partial.p, nv, w.sums.p + 3, w.stream), "reduce"); count(w);
     float tmax = 0;
     double d2[2] = {0, 0};
     cuda_check(cudaMemcpyAsync(&tmax, w.scalars_f.p + 1, sizeof(float), cudaMemcpyDeviceToHost, w.stream), "D2H");
@@ -834,7 +834,7 @@ void Solver::solve_batch(Work& w, BatchFeeder& feed) {
     NvtxRange range("solve_batch");
     cuda_check(cudaSetDevice(opts.device), "cudaSetDevice");
     const TileGeom g = geom();
-    const int nt = g.ntiles, K = w.k;
+    const int nv = vector_partials(g), K = w.k;
     const int mode = opts.precision_mode == HDD_PRECISION_MIXED ? 1 : 0;
     const int np = laplace_partials(g);
     const size_t N = w.vstride;
@@ -865,7 +865,7 @@ void Solver::solve_batch(Work& w, BatchFeeder& feed) {
     auto pds = [&](int j) { return w.partial.p + (size_t)j * w.pstride; };
     auto read_max = [&](int j, float* slot_out) {
         float v = 0;
-        cuda_check(launch_reduce_max(pms(j), nt, slot_out, w.stream), "reduce");
+        cuda_check(launch_reduce_max(pms(j), nv, slot_out, w.stream), "reduce");
         count(w);
         cuda_check(cudaMemcpyAsync(&v, slot_out, sizeof(float), cudaMemcpyDeviceToHost, w.stream), "D2H");
         sync(w);
@@ -879,11 +879,11 @@ void Solver::solve_batch(Work& w, BatchFeeder& feed) {
         if (mode == 1) cuda_check(launch_residual_f64(g, bs(j), xds(j), qs(j), pms(j), w.stream), "true residual");
         else cuda_check(launch_residual(g, bs(j), xs(j), qs(j), pms(j), w.stream), "true residual");
         count(w);
-        cuda_check(launch_reduce_max(pms(j), nt, sf + 1, w.stream), "reduce"); count(w);
+        cuda_check(launch_reduce_max(pms(j), nv, sf + 1, w.stream), "reduce"); count(w);
         cuda_check(launch_project_dot(g, qs(j), qs(j), pds(j), w.stream), "dot"); count(w);
-        cuda_check(launch_reduce_sum(pds(j), nt, w.sums.p + 8 * j + 2, w.stream), "reduce"); count(w);
+        cuda_check(launch_reduce_sum(pds(j), nv, w.sums.p + 8 * j + 2, w.stream), "reduce"); count(w);
         cuda_check(launch_project_dot(g, bs(j), bs(j), pds(j), w.stream), "dot"); count(w);
-        cuda_check(launch_reduce_sum(pds(j), nt, w.sums.p + 8 * j + 3, w.stream), "reduce"); count(w);
+        cuda_check(launch_reduce_sum(pds(j), nv, w.sums.p + 8 * j + 3, w.stream), "reduce"); count(w);
         float tmax = 0;
         double d2[2] = {0, 0};
         cuda_check(cudaMemcpyAsync(&tmax, sf + 1, sizeof(float), cudaMemcpyDeviceToHost, w.stream), "D2H");
@@ -994,7 +994,7 @@ void Solver::solve_batch(Work& w, BatchFeeder& feed) {
         const int first1 = K == 1 ? h_first[0] : 0;
         apply_preconditioner(w, w.r.p, w.z.p);
         cuda_check(launch_project_dot(g, w.z.p, w.r.p, w.partial.p, w.stream, B), "project_dot"); count(w);
-        cuda_check(launch_reduce_sum(w.partial.p, nt, w.sums.p + 0, w.stream, B, 8), "reduce"); count(w);
+        cuda_check(launch_reduce_sum(w.partial.p, nv, w.sums.p + 0, w.stream, B, 8), "reduce"); count(w);
         cuda_check(launch_scalar_rho(w.scal.p, w.sums.p + 0, first1, w.stream, B, 8), "rho"); count(w);
         cuda_check(launch_update_s(g, w.s.p, w.z.p, w.scal.p, first1, mode, w.stream, B), "update_s"); count(w);
         cuda_check(launch_laplace_dot(g, w.s.p, w.q.p, w.partial.p, w.stream, B), "laplace"); count(w);
@@ -1021,7 +1021,7 @@ void Solver::solve_batch(Work& w, BatchFeeder& feed) {
             cuda_check(launch_residual_f64(g, w.b.p, w.xd.p, w.r.p, w.partial_max.p, w.stream, R), "true residual");
             count(w);
         }
-        cuda_check(launch_reduce_max(w.partial_max.p, nt, w.scalars_f.p, w.stream, B, 8), "reduce"); count(w);
+        cuda_check(launch_reduce_max(w.partial_max.p, nv, w.scalars_f.p, w.stream, B, 8), "reduce"); count(w);
         for (int j = 0; j < K; ++j) {
             if (!sys[j].busy) continue;
             cuda_check(cudaMemcpyAsync(&h_rmax[j], w.scalars_f.p + 8 * j, sizeof(float), cudaMemcpyDeviceToHost,
