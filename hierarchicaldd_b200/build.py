@@ -29,6 +29,7 @@ SOURCES = [
     "kernels_pcg.cu",
     "sigma.cu",
     "sn_plan.cpp",
+    "sn_streams.cpp",
     "sn_solve.cu",
     "sn_resident.cu",
     "solver.cu",

@@ -55,7 +55,7 @@
 #include <vector>
 
 #include "dev_util.h"
-#include "sigma.h"
+#include "sn_streams.h"
 
 namespace hdd {
 namespace {
@@ -73,27 +73,6 @@ constexpr int kWarps = kNT / 32;
 constexpr int kTallRows = 512;
 __host__ __device__ constexpr int cols_of(int cw) { return kWarps * cw; }
 __host__ __device__ constexpr int rows_of(int cw) { return kBLoads / cw * 128; }
-// Partial sums a tree may need beside its unknowns.
-constexpr int kPartMax = 4096;
-// The trees one CTA takes of a cut plan: at most a cut of front_weight() and a
-// vector of kCutLen.  A front costs its coefficients and about what 1000
-// coefficients do for its operations (the trees of sparse domains are thousands
-// of tiny fronts).  The cut grows with the plan so that its trees are about one
-// CTA per SM: larger ones would take longer than the task levels they save,
-// smaller ones leave more of those.  Measured (us per
-// solve at cuts of total/280 and at least 16000, total/250 and 36000,
-// total/170 and 48000): interface of 40x36x44, sub 8 (9 MB) 82, 81, 75; 64^3,
-// sub 16 (15 MB) 86, 87, 84; second level of 192^3, sub 32 (39 MB) 94, 90, 101;
-// 128^3 (63 MB) 121, 124, 119; sparse 128^3 43, 41, 31.
-constexpr double kCutMin = 48000, kCutMax = 200000, kCutShare = 220;
-// One CTA per whole tree takes as long as its largest tree's weight; cut, about
-// as long as kCutCost, and a kCutRate-th of all.  Measured (us
-// per solve): 8 interiors of 32^3 whole 158, cut 69; 16, 32 and 48 of them cut
-// 81, 104 and 153; 64 whole 165; a 16^3 domain's interface (564 unknowns) whole
-// 27, cut 43.
-constexpr double kCutCost = 300000, kCutRate = 80;
-constexpr int kCutLen = 8192;
-
 struct PlanView {
     int nsn, n_fwd, ntasks;
     const int* rows;
@@ -445,71 +424,6 @@ __global__ void __launch_bounds__(kNT, kPerSM) sn_task_kernel(PlanView P) {
     }
 }
 
-double front_weight(const SnFactor& F, size_t j) {
-    return 1000.0 + 0.5 * F.ncol[j] * (F.ncol[j] + 1.0) + (double)F.rows[j].size() * F.ncol[j];
-}
-double tree_weight(const SnFactor& F) {
-    double w = 0;
-    for (size_t j = 0; j < F.col0.size(); ++j) w += front_weight(F, j);
-    return w;
-}
-
-// Plans solved by one CTA per factor (sn_resident.cu): every factor's unknowns
-// fit a CTA's shared memory, and cutting them would not pay.
-bool resident_plan(const std::vector<const SnFactor*>& factors, double total) {
-    int max_n = 0;
-    double largest = 0;
-    for (const SnFactor* F : factors) {
-        max_n = std::max(max_n, F->n);
-        largest = std::max(largest, tree_weight(*F));
-    }
-    if (max_n == 0 || ResidentPlan::smem_bytes(max_n + kPartMax, 1, 512) > ResidentPlan::kMaxSmem) return false;
-    return largest <= kCutCost + total / kCutRate;
-}
-
-// The lower trees of factor F (unknowns from `off` on, fronts from `base` on in
-// the plan): the largest subtrees of at most weight `cap`, each marked in low /
-// cut_root; consecutive ones share a CTA up to that weight.
-void cut_trees(const SnFactor& F, int off, int base, double cap, std::vector<char>& low, std::vector<char>& cut_root,
-               std::vector<ResidentPlan::Shape>& shapes, std::vector<int>& shape_off,
-               std::vector<std::vector<int>>& shape_roots) {
-    const int ns = (int)F.col0.size();
-    std::vector<double> weight(ns);
-    std::vector<int> size(ns, 1), len(ns);
-    for (int j = 0; j < ns; ++j) {
-        weight[j] += front_weight(F, j);
-        len[j] += F.ncol[j];
-        if (F.parent[j] >= 0) {
-            weight[F.parent[j]] += weight[j];
-            size[F.parent[j]] += size[j];
-            len[F.parent[j]] += len[j];
-        }
-    }
-    auto fits = [&](int j) { return weight[j] <= cap && (len[j] + (int)F.rows[j].size()) <= kCutLen; };
-    double w = 0;
-    int n = 0;
-    for (int j = 0; j < ns; ++j) {
-        if (!fits(j) || (F.parent[j] >= 0 && fits(F.parent[j]))) continue;
-        const int vec = len[j] + (int)F.rows[j].size();
-        if (shape_off.empty() || shapes.back().F != &F || shape_off.back() != off || w + weight[j] > cap ||
-            n + vec > kCutLen) {
-            shapes.emplace_back();
-            shapes.back().F = &F;
-            shapes.back().ext_off = off;
-            shape_off.push_back(off);
-            shape_roots.emplace_back();
-            w = 0;
-            n = 0;
-        }
-        w += weight[j];
-        n += vec;
-        shapes.back().trees.push_back({j - size[j] + 1, j, -1});
-        shape_roots.back().push_back(base + j);
-        cut_root[base + j] = 1;
-        for (int i = j - size[j] + 1; i <= j; ++i) low[base + i] = 1;
-    }
-}
-
 }  // namespace
 
 // Most unknowns a front above the trees may have rows and columns: each
@@ -562,7 +476,7 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
     std::vector<ResidentPlan::Shape> shapes;
     std::vector<int> shape_off;
     std::vector<std::vector<int>> shape_roots;  // plan fronts of the trees' roots
-    const double cap = std::min(kCutMax, std::max(kCutMin, total / kCutShare)) / shrink;
+    const double cap = cut_weight(total) / shrink;
     for (size_t f = 0; f < factors.size(); ++f)
         cut_trees(*factors[f], offsets[f], base[f], cap, low, cut_root, shapes, shape_off, shape_roots);
     // The fronts above, numbered in post-order, factor by factor.  Members given

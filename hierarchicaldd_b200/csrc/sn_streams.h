@@ -1,0 +1,150 @@
+// The schedule of solves with one CTA per elimination tree: the format of the
+// warps' streams that sn_resident.cu runs, and the host code that writes them
+// (sn_streams.cpp, without CUDA calls, so that CPU tests can walk a schedule).
+#pragma once
+#include <array>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include "sigma.h"
+
+#ifdef __CUDACC__
+#define HDD_HD __host__ __device__
+#else
+#define HDD_HD
+#endif
+
+namespace hdd {
+
+// Lines of one warp's stream from the class's first: forward, then backward.
+struct RWarp {
+    int first, nf, nb, pad;
+};
+// One CTA's work: `count` members of a class.
+struct RGroup {
+    long long stream;         // byte offset of the class's streams
+    long long upd, y;         // offsets of the group's scratch, in doubles
+    int n, perm;              // unknowns; offset of perm
+    int next, ext;            // unknowns of the plan above that cut trees read; offset of their indices
+    int warps;                // offset of the class's warps
+    int member0, count, pad;
+};
+
+constexpr int kLine = 512;              // bytes of a line: 16 a lane
+constexpr int kBatch = 4;               // lines copied, waited for and released together
+constexpr int kBatchBytes = kBatch * kLine;
+// Batches in flight per warp (K trees per CTA; the vectors of more leave less room).
+HDD_HD constexpr int depth_of(int k) { return k == 1 ? 4 : 2; }
+
+// Operations of a stream.  Each starts with a batch whose first line is the
+// header, an int4 for every lane: {type | log2 of the lanes on row quads << 4 |
+// flags << 8, count, index, distance}.
+enum : int {
+    kEnd = 0,
+    kNothing = 1,   // (a barrier)
+    // Items on 1 to 3 lines (count), one per lane: {index, first, second entry,
+    // 1 when the index is a slot (GS)}: M[index] += the two entries.
+    kAssemble = 2,
+    // A block of a front times its inputs: count groups of four steps (a batch
+    // each), index: the lane's first column (forward), distance: from a lane's
+    // column to its next.  Lines: destinations of four rows a lane; forward the
+    // rows' pairs of children's entries (16 bits each) and one item of an
+    // assembly before; backward the columns' indices for the first sixteen
+    // steps (eight 16-bit indices a lane and line), a batch of four more such
+    // lines following every further 32 steps.
+    kProduct = 3,
+    // Items on 1 to 3 lines: {first partial sum, destination, first, second
+    // entry}; index: slices, distance: between their partial sums.
+    kFinish = 4
+};
+constexpr int kBar = 1;        // CTA barrier after it
+constexpr int kPairs = 2;      // the rows have children's entries
+constexpr int kItem = 4;       // the product starts with an assembly
+constexpr int kTransposed = 8;
+constexpr int kTopRoot = 16;   // destinations -1 - entry are the plan above's update vectors
+// Indices are into the CTA's array M: the vector, rows outside cut trees, a
+// zero (a pair's missing entries), an unused entry (results of no row), partial
+// sums and, where they fit, update slots.  GS: slots are in global memory
+// instead (destination -1 - slot; a pair's entries are slots, slot 0 the zero).
+
+// One operation of a warp, before it is written.
+struct Op {
+    int type, flags;
+    int front, r0, rows, c0, c1, po;  // product; po: first of its partial sums (-1: not split)
+    int i0, i1;                       // assembly, finish: items
+    int nsl, stride;                  // finish
+    int batches() const;
+};
+
+struct ClassPlan {
+    int n = 0, slots = 0, part_len = 0;  // unknowns; update slots and partial sums at a time
+    int zero = 0, none = 0, part0 = 0;   // indices in M: the zero, the unused entry, the first partial sum
+    std::vector<int> perm, ext;
+    std::vector<int> fronts;             // the factor's fronts
+    std::vector<int> c0;                 // index of each front's first unknown
+    std::vector<std::vector<int>> idx;   // index of every row of each front
+    std::vector<std::vector<int>> dst;   // destination of every row of each front, forward (kSlot + slot: a slot)
+    // Children's entries of every row of each front: first slot (a row's are consecutive) and count.
+    std::vector<std::vector<int>> slot, cnt;
+    std::vector<char> root;              // whether the front's update vector belongs to the plan above
+    std::vector<std::array<int, 4>> items;
+    std::vector<std::vector<Op>> fwd, bwd;  // per warp
+    double coef = 0;                     // coefficients of one direction
+    int slot0 = 0;                       // index in M of slot 0 (negative: slots are in global memory)
+    // Entries of M without slots, and the reach of products past their columns.
+    int entries() const { return part0 + part_len; }
+    static constexpr int kReach = 128;
+};
+// While M is not laid out, slots are numbered from kSlot on and kZero is the zero.
+constexpr int kSlot = 0x20000000, kZero = 0x10000000;
+
+// Everything of a ResidentPlan that does not need the device.
+struct ResidentSchedule {
+    bool cut = false, global_slots = false;
+    int max_n = 0, km = 1, nt = 512;
+    int entries = 0;                     // doubles of a CTA's trees in shared memory
+    size_t smem = 0;                     // shared memory of a CTA
+    std::vector<RGroup> groups;
+    std::vector<RWarp> warps;
+    std::vector<int> off, perm, ext;
+    long long upd_len = 0, y_len = 0;    // doubles of the scratch
+    double coef = 0;                     // coefficients of one direction, each class's once
+    // Schedules shapes[c] for members[c] (offsets of their unknowns) on a device
+    // of nsm SMs; false when a CTA's shared memory does not hold the trees.
+    // The shapes are referred to until the streams are written.
+    bool plan(const std::vector<ResidentPlan::Shape>& shapes, const std::vector<std::vector<int>>& members, bool cut_trees,
+              int nsm);
+    // The streams, one per class and warp, in floats: `total` in all (padding
+    // that prefetches run into included), stream i from at(i) on.
+    size_t streams() const { return stream.size(); }
+    long long total() const;
+    long long at(size_t i) const { return stream[i].at; }
+    void write(size_t i, float* dst) const;
+
+private:
+    struct Item { int c, w; long long at; };
+    const std::vector<ResidentPlan::Shape>* shape = nullptr;
+    std::vector<ClassPlan> cp;
+    std::vector<Item> stream;            // the last: padding
+};
+
+// Whole factors: a shape per distinct factor, and its members' offsets.
+void whole_shapes(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets,
+                  std::vector<ResidentPlan::Shape>& shapes, std::vector<std::vector<int>>& members);
+
+// What a factor's trees weigh for the rules below.
+double tree_weight(const SnFactor& F);
+// Plans solved by one CTA per factor: every factor's unknowns fit a CTA's
+// shared memory, and cutting them would not pay.  total: all factors' weight.
+bool resident_plan(const std::vector<const SnFactor*>& factors, double total);
+// The heaviest tree cut from a plan of weight `total`.
+double cut_weight(double total);
+// The lower trees of factor F (unknowns from `off` on, fronts from `base` on in
+// the plan): the largest subtrees of at most weight `cap`, each marked in low /
+// cut_root; consecutive ones share a CTA up to that weight.
+void cut_trees(const SnFactor& F, int off, int base, double cap, std::vector<char>& low, std::vector<char>& cut_root,
+               std::vector<ResidentPlan::Shape>& shapes, std::vector<int>& shape_off,
+               std::vector<std::vector<int>>& shape_roots);
+
+}  // namespace hdd

@@ -18,7 +18,7 @@ def load_shim():
     os.makedirs(BUILD, exist_ok=True)
     srcs = [os.path.join(ROOT, "tests", "host_shim.cpp")] + [
         os.path.join(CSRC, f) for f in ("host_setup.cpp", "host_interface.cpp", "host_cholesky.cpp", "host_interface_io.cpp",
-                                        "sn_plan.cpp")]
+                                        "sn_plan.cpp", "sn_streams.cpp")]
     if not os.path.exists(SHIM) or any(os.path.getmtime(f) > os.path.getmtime(SHIM) for f in srcs):
         subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fopenmp", "-ffp-contract=off",
                         "-I", CSRC, "-I", os.path.join(ROOT, "include"), "-I", "/usr/local/cuda/include",
