@@ -212,7 +212,6 @@ struct ResidentPlan {
     bool cut = false;                   // cut trees: separate forward and backward launches
     int n = 0, max_n = 0, ngroups = 0;  // unknowns; largest vector; CTAs of one solve (0: no plan)
     int km = 1, nt = 256;               // trees per CTA (1, 2 or 4), threads per CTA
-    int entries = 0;                    // doubles of a CTA's trees in shared memory
     int resident = 1;                   // CTAs that fit on the device
     size_t smem = 0, bytes = 0;         // shared memory per CTA; device bytes
     long long upd_len = 0, y_len = 0;   // doubles of a ResidentScratch's buffers

@@ -64,7 +64,6 @@ struct RView {
     const double* top_x;
     long long ld_upd, ld_y, ld_top_upd, ld_top_x, ld_b, ld_x;
     int ngroups, nrhs;
-    int entries;                       // doubles of all of a CTA's Ms
     int* ctr;                          // forward: counters to clear
     long long n_ctr;
     const int* gate;                   // test seam: nonzero = wait for it to clear
@@ -206,7 +205,7 @@ __device__ __forceinline__ void four_steps(Stream<D>& S, const double* m, const 
 template <int K, int D, bool GS>
 __device__ __forceinline__ void op_product(Stream<D>& S, const Vec<K>& V, const int4 h, const int4 dst, const int4 p2,
                                            const int4 p3) {
-    const int lmq = (h.x >> 4) & 15, flags = h.x >> 8, groups = h.y;
+    const int lmq = (h.x >> 4) & 15, flags = (h.x >> 8) & 255, groups = h.x >> 16;
     double acc[K][4];
 #pragma unroll
     for (int k = 0; k < K; ++k)
@@ -241,15 +240,18 @@ __device__ __forceinline__ void op_product(Stream<D>& S, const Vec<K>& V, const 
         }
     } else {
         if (flags & kItem) {
-            assemble_item<K, GS>(V, p3);
+            if (p3.x >= 0) assemble_item<K, GS>(V, p3);
             __syncwarp();
         }
-        int c = h.z;
-        for (int g = 0; g < groups; ++g) {
-            const int j[4] = {c, c + h.w, c + 2 * h.w, c + 3 * h.w};
+        int c = h.y & 0xffff;
+        const int d = h.y >> 16;
+        for (int g = 1; g < groups; ++g) {
+            const int j[4] = {c, c + d, c + 2 * d, c + 3 * d};
             four_steps<K, D>(S, V.m, j, acc);
-            c += 4 * h.w;
+            c += 4 * d;
         }
+        const int j[4] = {h.z & 0xffff, (int)((uint32_t)h.z >> 16), h.w & 0xffff, (int)((uint32_t)h.w >> 16)};
+        four_steps<K, D>(S, V.m, j, acc);
     }
     // The column slices, summed by a fixed shuffle tree.
 #pragma unroll
@@ -307,18 +309,18 @@ __device__ __forceinline__ void run_stream(Stream<D>& S, const Vec<K>& V) {
         const int4 h = S.template line<int4>(0), l1 = S.template line<int4>(1), l2 = S.template line<int4>(2),
                    l3 = S.template line<int4>(3);
         S.pop();
-        const int type = h.x & 15;
+        const int type = h.x & 15, count = h.x >> 16;
         if (type == kProduct) {
             op_product<K, D, GS>(S, V, h, l1, l2, l3);
         } else if (type == kAssemble) {
             if (l1.x >= 0) assemble_item<K, GS>(V, l1);
-            if (h.y > 1 && l2.x >= 0) assemble_item<K, GS>(V, l2);
-            if (h.y > 2 && l3.x >= 0) assemble_item<K, GS>(V, l3);
+            if (count > 1 && l2.x >= 0) assemble_item<K, GS>(V, l2);
+            if (count > 2 && l3.x >= 0) assemble_item<K, GS>(V, l3);
         } else if (type == kFinish) {
             const bool top = (h.x >> 8) & kTopRoot;
-            if (l1.x >= 0) finish_item<K, GS>(V, l1, h.z, h.w, top);
-            if (h.y > 1 && l2.x >= 0) finish_item<K, GS>(V, l2, h.z, h.w, top);
-            if (h.y > 2 && l3.x >= 0) finish_item<K, GS>(V, l3, h.z, h.w, top);
+            if (l1.x >= 0) finish_item<K, GS>(V, l1, h.y, h.z, top);
+            if (count > 1 && l2.x >= 0) finish_item<K, GS>(V, l2, h.y, h.z, top);
+            if (count > 2 && l3.x >= 0) finish_item<K, GS>(V, l3, h.y, h.z, top);
         } else if (type == kEnd) {
             return;
         }
@@ -413,10 +415,6 @@ template <int KM, int NT, int MODE, bool GS>
 __global__ void __launch_bounds__(NT, resident_min_blocks(NT))
     sn_resident_kernel(RView P, const float* __restrict__ b_old, float* __restrict__ x_old) {
     extern __shared__ __align__(16) char smem[];
-    // Products read past a front's columns (times zero): no NaN may be there.
-    double* m = reinterpret_cast<double*>(smem + (size_t)(NT / 32) * depth_of(KM) * kBatchBytes);
-    for (int i = threadIdx.x; i < P.entries; i += NT) m[i] = 0.0;
-    __syncthreads();
     for (int w = blockIdx.x; w < P.ngroups * P.nrhs; w += gridDim.x) {
         const RGroup G = P.groups[w / P.nrhs];
         const int rhs = w % P.nrhs;
@@ -504,7 +502,6 @@ bool ResidentPlan::build_shapes(const std::vector<Shape>& shapes, const std::vec
     max_n = S.max_n;
     km = S.km;
     nt = S.nt;
-    entries = S.entries;
     smem = S.smem;
     global_slots = S.global_slots;
     ngroups = (int)S.groups.size();
@@ -557,7 +554,7 @@ void ResidentPlan::launch(int mode, const ResidentScratch& sc, const TopVectors&
                           long long spin_limit, const float* b_old, float* x_old, cudaStream_t s, int nrhs,
                           long long ld_b, long long ld_x) const {
     const RView P{d_groups, d_warps, d_off, d_perm, d_ext, d_stream, sc.upd, sc.y, top.upd, top.x,
-                  upd_len, y_len, top.ld_upd, top.ld_x, ld_b, ld_x, ngroups, nrhs, entries, top.ctr, top.n_ctr, d_gate, err,
+                  upd_len, y_len, top.ld_upd, top.ld_x, ld_b, ld_x, ngroups, nrhs, top.ctr, top.n_ctr, d_gate, err,
                   spin_limit};
     const int all = ngroups * nrhs;
     const int grid = grid_div > 1 ? std::min(all, std::max(1, (resident + grid_div - 1) / grid_div)) : all;

@@ -419,12 +419,11 @@ uint32_t* emit(const Op& o, const SnFactor& F, const ClassPlan& P, uint32_t* out
     auto place = [&](int d) { return d < kZero ? d : (gs ? -1 - (1 + d - kSlot) : P.slot0 + d - kSlot); };
     // Entries of pairs: in M, or slots of global memory after its zero.
     auto entry = [&](int d) { return d == kZero ? (gs ? 0 : P.zero) : (gs ? 1 : P.slot0) + d - kSlot; };
-    auto header = [&](int lmq, int count, auto index, int distance) {
+    auto header = [&](int lmq, int count, int a = 0, int b = 0) {
         for (int l = 0; l < 32; ++l) {
-            h[4 * l] = o.type | lmq << 4 | o.flags << 8;
-            h[4 * l + 1] = count;
-            h[4 * l + 2] = index(l);
-            h[4 * l + 3] = distance;
+            h[4 * l] = o.type | lmq << 4 | o.flags << 8 | count << 16;
+            h[4 * l + 1] = a;
+            h[4 * l + 2] = b;
         }
     };
     auto assemble_entry = [&](int* p, const std::array<int, 4>& t) {
@@ -436,7 +435,7 @@ uint32_t* emit(const Op& o, const SnFactor& F, const ClassPlan& P, uint32_t* out
     };
     if (o.type != kProduct) {
         const int n = o.i1 - o.i0;
-        header(0, (n + 31) / 32, [&](int) { return o.nsl; }, o.stride);
+        header(0, (n + 31) / 32, o.nsl, o.stride);
         int* p = h + L;
         for (int i = 0; i < kItems; ++i, p += 4) {
             if (i >= n) {
@@ -459,7 +458,17 @@ uint32_t* emit(const Op& o, const SnFactor& F, const ClassPlan& P, uint32_t* out
     const int i = o.front, m = (int)P.idx[i].size();
     const int lmq = log2_lanes(o.rows), mq = 1 << lmq, ns = 32 >> lmq;
     const int groups = groups_of(o.rows, o.c1 - o.c0);
-    header(lmq, groups, [&](int l) { return tr ? 0 : P.c0[i] + o.c0 + (l >> lmq); }, ns);
+    header(lmq, groups);
+    // The index of a lane's step: past the block's columns the zero.
+    auto input = [&](int l, int step) {
+        const int c = o.c0 + (l >> lmq) + step * ns;
+        return c < o.c1 ? P.idx[i][c] : P.zero;
+    };
+    if (!tr)
+        for (int l = 0; l < 32; ++l) {
+            h[4 * l + 1] = (P.c0[i] + o.c0 + (l >> lmq)) | ns << 16;
+            for (int u = 0; u < 4; ++u) h[4 * l + 2 + u / 2] |= input(l, 4 * (groups - 1) + u) << (u % 2 * 16);
+        }
     auto rows_line = [&](int line, auto value) {  // one int per row, four a lane (the first slice's lanes)
         int* p = h + line * L;
         for (int l = 0; l < 32; ++l)
@@ -485,19 +494,14 @@ uint32_t* emit(const Op& o, const SnFactor& F, const ClassPlan& P, uint32_t* out
         int* p = h + 3 * L;
         for (int l = 0; l < 32; ++l, p += 4) {
             if (o.i0 + l < o.i1) assemble_entry(p, P.items[o.i0 + l]);
-            else {  // adds zero to the unused entry
-                p[0] = P.none;
-                p[1] = p[2] = entry(kZero);
-                p[3] = 0;
-            }
+            else p[0] = -1;
         }
     }
     // Eight steps' column indices, 16 bits each.
     auto index_line = [&](uint32_t* line, int step0) {
         uint16_t* p = reinterpret_cast<uint16_t*>(line);
         for (int l = 0; l < 32; ++l)
-            for (int u = 0; u < 8; ++u)
-                p[8 * l + u] = (uint16_t)P.idx[i][std::min(o.c1 - 1, o.c0 + (l >> lmq) + (step0 + u) * ns)];
+            for (int u = 0; u < 8; ++u) p[8 * l + u] = (uint16_t)input(l, step0 + u);
     };
     if (tr) {
         index_line(out + 2 * L, 0);
@@ -601,16 +605,16 @@ bool ResidentSchedule::plan(const std::vector<ResidentPlan::Shape>& shapes,
     // M's entries with and without the update slots; trees per CTA.
     int bare = 0, all = 0;
     for (const ClassPlan& P : cp) {
-        bare = std::max(bare, P.entries() + ClassPlan::kReach);
-        all = std::max(all, P.entries() + std::max(P.slots, (int)ClassPlan::kReach));
+        bare = std::max(bare, P.entries());
+        all = std::max(all, P.entries() + P.slots);
     }
     km = 1;
     while (!cut && km < 4 && groups_for(km) > (size_t)nsm &&
            ResidentPlan::smem_bytes(bare, 2 * km, nt) <= ResidentPlan::kMaxSmem)
         km *= 2;
     global_slots = !cut && (ResidentPlan::smem_bytes(all, km, nt) > ResidentPlan::kMaxSmem || all >= 65536);
-    entries = (global_slots ? bare : all) * km;
-    smem = ResidentPlan::smem_bytes(global_slots ? bare : all, km, nt);
+    entries = global_slots ? bare : all;
+    smem = ResidentPlan::smem_bytes(entries, km, nt);
     bool fits = smem <= ResidentPlan::kMaxSmem;
     for (ClassPlan& P : cp) {
         P.slot0 = global_slots ? -1 : P.entries();

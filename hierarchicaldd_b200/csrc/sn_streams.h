@@ -39,7 +39,7 @@ HDD_HD constexpr int depth_of(int k) { return k == 1 ? 4 : 2; }
 
 // Operations of a stream.  Each starts with a batch whose first line is the
 // header, an int4 for every lane: {type | log2 of the lanes on row quads << 4 |
-// flags << 8, count, index, distance}.
+// flags << 8 | count << 16, and three more words of the type}.
 enum : int {
     kEnd = 0,
     kNothing = 1,   // (a barrier)
@@ -47,15 +47,18 @@ enum : int {
     // 1 when the index is a slot (GS)}: M[index] += the two entries.
     kAssemble = 2,
     // A block of a front times its inputs: count groups of four steps (a batch
-    // each), index: the lane's first column (forward), distance: from a lane's
-    // column to its next.  Lines: destinations of four rows a lane; forward the
-    // rows' pairs of children's entries (16 bits each) and one item of an
-    // assembly before; backward the columns' indices for the first sixteen
+    // each).  Header, forward: the lane's first column | distance to its next
+    // << 16, and the indices of the last group's four steps (16 bits each).
+    // Lines: destinations of four rows a lane; forward the rows' pairs of
+    // children's entries (16 bits each) and one item of an assembly before
+    // (index -1: none); backward the columns' indices for the first sixteen
     // steps (eight 16-bit indices a lane and line), a batch of four more such
-    // lines following every further 32 steps.
+    // lines following every further 32 steps.  Steps past the block's columns
+    // read the zero: what lies behind them may be another system's NaN or
+    // written by another warp, and zero coefficients do not undo a NaN.
     kProduct = 3,
     // Items on 1 to 3 lines: {first partial sum, destination, first, second
-    // entry}; index: slices, distance: between their partial sums.
+    // entry}.  Header: slices, distance between their partial sums.
     kFinish = 4
 };
 constexpr int kBar = 1;        // CTA barrier after it
@@ -64,8 +67,8 @@ constexpr int kItem = 4;       // the product starts with an assembly
 constexpr int kTransposed = 8;
 constexpr int kTopRoot = 16;   // destinations -1 - entry are the plan above's update vectors
 // Indices are into the CTA's array M: the vector, rows outside cut trees, a
-// zero (a pair's missing entries), an unused entry (results of no row), partial
-// sums and, where they fit, update slots.  GS: slots are in global memory
+// zero (a pair's missing entries), an unused entry (results of no row, never
+// read), partial sums and, where they fit, update slots.  GS: slots are in global memory
 // instead (destination -1 - slot; a pair's entries are slots, slot 0 the zero).
 
 // One operation of a warp, before it is written.
@@ -92,9 +95,7 @@ struct ClassPlan {
     std::vector<std::vector<Op>> fwd, bwd;  // per warp
     double coef = 0;                     // coefficients of one direction
     int slot0 = 0;                       // index in M of slot 0 (negative: slots are in global memory)
-    // Entries of M without slots, and the reach of products past their columns.
-    int entries() const { return part0 + part_len; }
-    static constexpr int kReach = 128;
+    int entries() const { return part0 + part_len; }  // of M, without slots
 };
 // While M is not laid out, slots are numbered from kSlot on and kZero is the zero.
 constexpr int kSlot = 0x20000000, kZero = 0x10000000;
@@ -103,7 +104,7 @@ constexpr int kSlot = 0x20000000, kZero = 0x10000000;
 struct ResidentSchedule {
     bool cut = false, global_slots = false;
     int max_n = 0, km = 1, nt = 512;
-    int entries = 0;                     // doubles of a CTA's trees in shared memory
+    int entries = 0;                     // entries of M
     size_t smem = 0;                     // shared memory of a CTA
     std::vector<RGroup> groups;
     std::vector<RWarp> warps;

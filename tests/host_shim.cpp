@@ -6,12 +6,14 @@
 #include <cstdint>
 #include <cstring>
 #include <exception>
+#include <functional>
+#include <limits>
 #include <random>
 #include <string>
 #include <vector>
 
 #include "host_setup.h"
-#include "sigma.h"
+#include "sn_streams.h"
 
 using namespace hdd;
 
@@ -29,6 +31,215 @@ const CsrF* pick(Shim* s, int kind, int level, int sub) {
         case 2: return (sub >= 0 && sub < s->ih.n_sub) ? &s->ih.Air[level][sub] : nullptr;
         case 3: return level < (int)s->ih.Prr.size() ? &s->ih.Prr[level] : nullptr;
         default: return nullptr;
+    }
+}
+
+// Walks a schedule of one CTA per tree the way sn_resident.cu runs it, one warp
+// after another between two barriers, with every index checked.  The CTA's
+// array M starts as NaN (what another system may have left there).
+struct StreamWalk {
+    const ResidentSchedule& S;
+    std::vector<float> words;      // the streams
+    long long oob = 0, races = 0;  // accesses out of range; of entries another warp uses in the same phase
+    long long ops = 0, barriers = 0;
+    explicit StreamWalk(const ResidentSchedule& s) : S(s), words((size_t)s.total()) {
+        for (size_t i = 0; i < S.streams(); ++i) S.write(i, words.data() + S.at(i));
+    }
+    int word(long long line, int i) const {
+        int v;
+        std::memcpy(&v, &words.at((size_t)(line * (kLine / 4) + i)), 4);
+        return v;
+    }
+    // Entries of M (or update slots in global memory) with their last users.
+    struct Memory {
+        std::vector<double> v;
+        std::vector<int> wp, ww, rp, rw;  // phase and warp of the last write / read (warp -2: several)
+        int free_entry = -1;              // results of no row: written by anyone, read by nobody
+        StreamWalk* walk = nullptr;
+        double dummy = 0;
+        void init(StreamWalk* s, long long n) {
+            walk = s;
+            v.assign((size_t)n, std::numeric_limits<double>::quiet_NaN());
+            wp.assign((size_t)n, -1); ww.assign((size_t)n, -1); rp.assign((size_t)n, -1); rw.assign((size_t)n, -1);
+        }
+        double read(long long i, int warp, int phase) {
+            if (i < 0 || i >= (long long)v.size() || i == free_entry) { ++walk->oob; return 0; }
+            if (wp[i] == phase && ww[i] != warp) ++walk->races;
+            rw[i] = rp[i] == phase && rw[i] != warp ? -2 : warp;
+            rp[i] = phase;
+            return v[i];
+        }
+        void write(long long i, double x, int warp, int phase) {
+            if (i < 0 || i >= (long long)v.size()) { ++walk->oob; return; }
+            if (i == free_entry) return;
+            if ((wp[i] == phase && ww[i] != warp) || (rp[i] == phase && rw[i] != warp)) ++walk->races;
+            wp[i] = phase;
+            ww[i] = warp;
+            v[i] = x;
+        }
+    };
+    // mode: 0 whole trees, 1 / 2 the forward / backward half of cut ones.
+    void run(int mode, const float* b, float* x, std::vector<double>& y, std::vector<double>& top_upd,
+             const std::vector<double>& top_x) {
+        const int nw = S.nt / 32;
+        for (const RGroup& G : S.groups)
+            for (int k = 0; k < G.count; ++k) {  // members side by side never meet
+                const int off = S.off.at(G.member0 + k);
+                const int zero = G.n + G.next;
+                Memory M, U;
+                M.init(this, S.entries);
+                M.free_entry = zero + 1;
+                U.init(this, S.global_slots ? 65536 : 0);
+                auto at = [&](long long i, int w, int p) { return M.read(i, w, p); };
+                auto slot = [&](long long i, int w, int p) { return S.global_slots ? U.read(i, w, p) : M.read(i, w, p); };
+                auto put = [&](int d, double v, int flags, int w, int p) {
+                    if (d >= 0) {
+                        if (d == zero) ++oob;
+                        M.write(d, v, w, p);
+                    } else if (S.global_slots) {
+                        if (d == -1) ++oob;  // the zero slot
+                        U.write(-1 - d, v, w, p);
+                    } else if ((flags & kTopRoot) && mode == 1 && -1 - d < (int)top_upd.size()) {
+                        top_upd[-1 - d] = v;
+                    } else {
+                        ++oob;
+                    }
+                };
+                auto assemble = [&](const int it[4], int w, int p) {
+                    const double s = slot(it[1], w, p) + slot(it[2], w, p);
+                    if (it[3] && S.global_slots) U.write(it[0], U.read(it[0], w, p) + s, w, p);
+                    else M.write(it[0], at(it[0], w, p) + s, w, p);
+                };
+                int phase = 0;
+                M.write(zero, 0.0, -1, phase);
+                if (S.global_slots) U.write(0, 0.0, -1, phase);
+                for (int i = 0; i < G.n; ++i)
+                    M.write(i, mode == 2 ? y.at(G.y + i) : (double)b[off + S.perm.at(G.perm + i)], -1, phase);
+                if (mode == 2)
+                    for (int i = 0; i < G.next; ++i) M.write(G.n + i, top_x.at(S.ext.at(G.ext + i)), -1, phase);
+                for (int pass = mode == 2 ? 1 : 0; pass < (mode == 1 ? 1 : 2); ++pass) {
+                    ++phase;
+                    std::vector<long long> pos(nw), lim(nw);
+                    std::vector<int> owed(nw, 0);  // barriers a warp has still to take
+                    for (int w = 0; w < nw; ++w) {
+                        const RWarp W = S.warps.at(G.warps + w);
+                        pos[w] = G.stream / kLine + W.first + (pass ? W.nf : 0);
+                        lim[w] = pos[w] + (pass ? W.nb : W.nf);
+                        // Copies run ahead by the ring's depth.
+                        if ((lim[w] + (long long)kBatch * depth_of(S.km)) * kLine > (long long)words.size() * 4) ++oob;
+                    }
+                    for (int ended = 0; ended < nw; ++phase) {
+                        ended = 0;
+                        int waiting = 0;
+                        for (int w = 0; w < nw; ++w) {
+                            if (owed[w] > 0) { --owed[w]; ++waiting; continue; }
+                            for (;;) {
+                                if (pos[w] >= lim[w]) { ++oob; ++ended; break; }
+                                const long long h = pos[w];
+                                const int type = word(h, 0) & 15, flags = (word(h, 0) >> 8) & 255;
+                                if (type == kEnd) {
+                                    if (h + kBatch != lim[w]) ++oob;
+                                    ++ended;
+                                    break;
+                                }
+                                ++ops;
+                                pos[w] = operation(h, w, phase, M, at, slot, put, assemble);
+                                if (flags & kBar) { ++waiting; break; }
+                            }
+                        }
+                        if (waiting > 0 && ended > 0) { ++oob; break; }  // warps at different barriers
+                        if (waiting > 0) ++barriers;
+                    }
+                }
+                if (mode == 1)
+                    for (int i = 0; i < G.n; ++i) y.at(G.y + i) = M.v[i];
+                else
+                    for (int i = 0; i < G.n; ++i) x[off + S.perm.at(G.perm + i)] = (float)M.v[i];
+            }
+    }
+    // One operation from line h on; returns the line behind it.
+    template <class At, class Slot, class Put, class Assemble>
+    long long operation(long long h, int w, int p, Memory& M, At at, Slot slot, Put put, Assemble assemble) {
+        const int type = word(h, 0) & 15, lmq = (word(h, 0) >> 4) & 15, flags = (word(h, 0) >> 8) & 255;
+        const int count = word(h, 0) >> 16;
+        auto item = [&](long long line, int l, int it[4]) {
+            for (int q = 0; q < 4; ++q) it[q] = word(line, 4 * l + q);
+            return it[0] >= 0;
+        };
+        int it[4];
+        if (type == kAssemble || type == kFinish) {
+            for (int q = 1; q <= count; ++q)
+                for (int l = 0; l < 32; ++l) {
+                    if (!item(h + q, l, it)) continue;
+                    if (type == kAssemble) { assemble(it, w, p); continue; }
+                    double t = at(it[0], w, p);
+                    for (int s = 1; s < word(h, 1); ++s) t += at(it[0] + s * word(h, 2), w, p);
+                    put(it[1], (slot(it[2], w, p) + slot(it[3], w, p)) + t, flags, w, p);
+                }
+            return h + kBatch;
+        }
+        if (type != kProduct) {
+            if (type != kNothing) ++oob;
+            return h + kBatch;
+        }
+        const int mq = 1 << lmq;
+        const bool tr = (flags & kTransposed) != 0;
+        if (flags & kItem)
+            for (int l = 0; l < 32; ++l)
+                if (item(h + 3, l, it)) assemble(it, w, p);
+        auto half = [](int v, int q) { return q ? (int)((uint32_t)v >> 16) : v & 0xffff; };
+        std::vector<double> acc(128, 0.0);
+        long long pos = h + kBatch, ix = h + 2;
+        for (int g = 0; g < count; ++g) {
+            if (tr && g >= 4 && (g - 4) % 8 == 0) { ix = pos; pos += kBatch; }
+            const int s0 = 4 * (g < 4 ? g : (g - 4) % 8);
+            for (int u = 0; u < 4; ++u, ++pos)
+                for (int l = 0; l < 32; ++l) {
+                    int j;
+                    if (tr) j = half(word(ix + (s0 + u) / 8, 4 * l + (s0 + u) % 8 / 2), u % 2);
+                    else if (g + 1 == count) j = half(word(h, 4 * l + 2 + u / 2), u % 2);
+                    else j = half(word(h, 4 * l + 1), 0) + (4 * g + u) * half(word(h, 4 * l + 1), 1);
+                    const double in = at(j, w, p);
+                    for (int e = 0; e < 4; ++e)
+                        acc[4 * l + e] = std::fma((double)words.at((size_t)(pos * (kLine / 4) + 4 * l + e)), in, acc[4 * l + e]);
+                }
+        }
+        for (int o = 4; o < 32; o <<= 1)
+            if (mq <= o) {
+                const std::vector<double> a = acc;
+                for (int l = 0; l < 32; ++l)
+                    for (int e = 0; e < 4; ++e) acc[4 * l + e] = a[4 * l + e] + a[4 * (l ^ o) + e];
+            }
+        for (int l = 0; l < mq; ++l)
+            for (int e = 0; e < 4; ++e) {
+                double v = acc[4 * l + e];
+                if (flags & kPairs) {
+                    const int a = word(h + 2, 4 * l + e);
+                    v = (slot(half(a, 0), w, p) + slot(half(a, 1), w, p)) + v;
+                }
+                put(word(h + 1, 4 * l + e), v, flags, w, p);
+            }
+        return pos;
+    }
+};
+
+// The factors of one interface solve with their offsets, as the sigma solver
+// passes them to a plan (subdomains with equal systems share a factor).
+void plan_factors(const InterfaceHost& ih, int kind, int level, std::vector<SnFactor>& store,
+                  std::vector<const SnFactor*>& fs, std::vector<int>& offs) {
+    PlanHost ph;
+    interface_solve_plan(ih, kind, level, store, ph);
+    if (kind == 0) {
+        fs.push_back(&store[0]);
+        offs.push_back(0);
+        return;
+    }
+    const std::vector<int> rep = interior_classes(ih, level);
+    int off = 0;
+    for (int sd = 0; sd < ih.n_sub; ++sd) {
+        const int n = ih.Aii[level][sd].rows;
+        if (n > 0) { fs.push_back(&store[rep[sd]]); offs.push_back(off); }
+        off += n;
     }
 }
 }  // namespace
@@ -365,6 +576,122 @@ int shim_plan_emulate(void* h, int kind, int level, const float* b, float* x) {
         PlanHost plan;
         interface_solve_plan(s->ih, kind, level, fs, plan);
         plan.emulate(b, x);
+        return 0;
+    } catch (const std::exception&) {
+        return 1;
+    }
+}
+
+// The same solve through the schedule the device runs (sn_streams.h): whole
+// trees, or the lower trees of every factor with the fronts above them solved
+// front by front.  info: {1 whole / 0 cut, trees per CTA, threads per CTA, 1 when
+// update slots are in global memory, CTAs, fronts above, accesses out of range,
+// races between warps, operations, barriers}; *bytes: of the streams, *coef: the
+// distinct coefficients' of both directions.  Returns 0, or 1 on an exception.
+int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int* info, double* bytes, double* coef) {
+    try {
+        const InterfaceHost& ih = static_cast<Shim*>(h)->ih;
+        if (level < 0 || level >= ih.M || (kind != 0 && kind != 1)) return 1;
+        std::vector<SnFactor> store;
+        std::vector<const SnFactor*> fs;
+        std::vector<int> offs;
+        plan_factors(ih, kind, level, store, fs, offs);
+        double total = 0;
+        for (const SnFactor* F : fs) total += tree_weight(*F);
+        std::vector<ResidentPlan::Shape> shapes;
+        std::vector<std::vector<int>> members;
+        std::vector<double> y, upd, sol;
+        ResidentSchedule S;
+        constexpr int kSMs = 148;
+        bool whole = resident_plan(fs, total);
+        if (whole) {
+            whole_shapes(fs, offs, shapes, members);
+            whole = S.plan(shapes, members, false, kSMs);
+        }
+        int ntop = 0;
+        std::vector<long long> counts(4, 0);
+        auto done = [&](const StreamWalk& W) {
+            const int v[10] = {whole ? 1 : 0, S.km, S.nt, S.global_slots ? 1 : 0, (int)S.groups.size(), ntop,
+                               (int)W.oob, (int)W.races, (int)W.ops, (int)W.barriers};
+            std::copy(v, v + 10, info);
+            *bytes = 4.0 * S.total();
+            *coef = 8.0 * S.coef;
+        };
+        if (whole) {
+            StreamWalk W(S);
+            W.run(0, b, x, y, upd, sol);
+            done(W);
+            return 0;
+        }
+        std::vector<int> base(fs.size() + 1, 0), shape_off;
+        for (size_t f = 0; f < fs.size(); ++f) base[f + 1] = base[f] + (int)fs[f]->col0.size();
+        std::vector<char> low(base.back(), 0), root(base.back(), 0);
+        std::vector<std::vector<int>> roots;
+        for (size_t f = 0; f < fs.size(); ++f)
+            cut_trees(*fs[f], offs[f], base[f], cut_weight(total), low, root, shapes, shape_off, roots);
+        // Update vectors of the fronts above and of the trees' roots.
+        std::vector<int> at(base.back(), -1);
+        for (size_t f = 0; f < fs.size(); ++f)
+            for (size_t j = 0; j < fs[f]->col0.size(); ++j)
+                if (!low[base[f] + j] || root[base[f] + j]) {
+                    at[base[f] + j] = (int)upd.size();
+                    upd.resize(upd.size() + fs[f]->rows[j].size(), std::numeric_limits<double>::quiet_NaN());
+                }
+        for (size_t i = 0; i < shapes.size(); ++i)
+            for (size_t t = 0; t < shapes[i].trees.size(); ++t)
+                if (!shapes[i].F->rows[shapes[i].trees[t].last].empty()) shapes[i].trees[t].top = at[roots[i][t]];
+        for (int o : shape_off) members.push_back({o});
+        S = ResidentSchedule();
+        if (!S.plan(shapes, members, true, kSMs)) return 1;
+        StreamWalk W(S);
+        y.assign((size_t)S.y_len, 0.0);
+        W.run(1, b, x, y, upd, sol);
+        int n = 0;
+        for (size_t f = 0; f < fs.size(); ++f) n = std::max(n, offs[f] + fs[f]->n);
+        sol.assign(n, 0.0);
+        for (size_t f = 0; f < fs.size(); ++f) {
+            const SnFactor& F = *fs[f];
+            const int ns = (int)F.col0.size();
+            std::vector<std::vector<int>> kids(ns);
+            for (int j = 0; j < ns; ++j)
+                if (F.parent[j] >= 0) kids[F.parent[j]].push_back(j);
+            std::vector<std::vector<double>> yv(ns);
+            for (int j = 0; j < ns; ++j) {
+                if (low[base[f] + j]) continue;
+                ++ntop;
+                const int nj = F.ncol[j], nr = (int)F.rows[j].size(), m = nj + nr;
+                std::vector<double> v(m, 0.0);
+                for (int a = 0; a < nj; ++a) v[a] = b[offs[f] + F.perm[F.col0[j] + a]];
+                for (int c : kids[j])
+                    for (size_t q = 0; q < F.rows[c].size(); ++q) {
+                        const int r = F.rows[c][q];
+                        const int i = r < F.col0[j] + nj ? r - F.col0[j]
+                                                         : nj + (int)(std::lower_bound(F.rows[j].begin(), F.rows[j].end(), r) -
+                                                                      F.rows[j].begin());
+                        v[i] += upd[at[base[f] + c] + q];
+                    }
+                for (int r = 0; r < m; ++r) {
+                    double s = 0;
+                    for (int c = 0; c < nj; ++c) s += (double)(float)F.Fw[j][(size_t)c * m + r] * v[c];
+                    if (r < nj) yv[j].push_back(s);
+                    else upd[at[base[f] + j] + r - nj] = v[r] + s;
+                }
+            }
+            for (int j = ns - 1; j >= 0; --j) {
+                if (low[base[f] + j]) continue;
+                const int nj = F.ncol[j], m = nj + (int)F.rows[j].size();
+                for (int a = 0; a < nj; ++a) {
+                    double s = 0;
+                    for (int r = 0; r < m; ++r)
+                        s += (double)(float)F.Fw[j][(size_t)a * m + r] *
+                             (r < nj ? yv[j][r] : sol[offs[f] + F.rows[j][r - nj]]);
+                    sol[offs[f] + F.col0[j] + a] = s;
+                    x[offs[f] + F.perm[F.col0[j] + a]] = (float)s;
+                }
+            }
+        }
+        W.run(2, b, x, y, upd, sol);
+        done(W);
         return 0;
     } catch (const std::exception&) {
         return 1;

@@ -1,0 +1,58 @@
+"""The schedules of the one-CTA-per-tree solves (sn_streams.cpp), walked on the
+CPU operation by operation as sn_resident.cu runs them: against the host walk of
+the same fronts, from a CTA's array that holds NaN everywhere (a system that
+broke down may have left it so: nothing a solve has not written itself may reach
+its result), with every index in range and no entry written by one warp that
+another warp reads or writes before the next barrier.
+
+Tolerance as for the kernels: FP64 sums in another order, rounded to FP32 once,
+one ulp (1.2e-7) of the largest entry.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from shim_ffi import load_shim
+from sn_routes import ROUTES, domain
+
+RTOL = 1.2e-7
+
+
+def _fp(a):
+    return a.ctypes.data_as(C.POINTER(C.c_float))
+
+
+def _unknowns(shim, h, kind, level):
+    shape = (C.c_int * 3)()
+    subs = range(shim.shim_num_subdomains(h)) if kind else [0]
+    return sum(shape[0] for i in subs if shim.shim_matrix_shape(h, kind, level, i, shape) == 0)
+
+
+@pytest.mark.parametrize("name", ROUTES)
+def test_schedules_read_nothing_but_their_own_system(name):
+    d, levels = domain(name)
+    shim = load_shim()
+    err = C.create_string_buffer(512)
+    flags = np.ascontiguousarray(d.flags, np.uint32)
+    h = shim.shim_build((C.c_int * 3)(*d.size), (C.c_int * 3)(*d.sub_size), d.meta["vlevels"], levels,
+                        flags.ctypes.data_as(C.POINTER(C.c_uint32)), err, 512)
+    assert h, err.value
+    rng = np.random.default_rng(3)
+    try:
+        for level in range(levels):
+            for kind in (0, 1):
+                n = _unknowns(shim, h, kind, level)
+                if n == 0:
+                    continue
+                b = rng.uniform(-1, 1, n).astype(np.float32)
+                x, xe = np.full(n, np.nan, np.float32), np.zeros(n, np.float32)
+                info, by, co = (C.c_int * 10)(), C.c_double(), C.c_double()
+                assert shim.shim_stream_walk(h, kind, level, _fp(b), _fp(x), info, C.byref(by), C.byref(co)) == 0
+                assert shim.shim_plan_emulate(h, kind, level, _fp(b), _fp(xe)) == 0
+                assert info[6] == 0 and info[7] == 0, (level, kind, "out of range, races", info[6], info[7])
+                assert np.all(np.isfinite(x)), (level, kind, "NaN from outside the system")
+                diff = float(np.max(np.abs(x.astype(np.float64) - xe)))
+                assert diff <= RTOL * float(np.max(np.abs(xe))), (level, kind, diff)
+    finally:
+        shim.shim_free(h)

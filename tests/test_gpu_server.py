@@ -228,3 +228,30 @@ def test_batched_requests_equal_solo_solves(batch, precision):
         assert srv.memory()[0] == 0
     finally:
         srv.close()
+
+
+@pytest.mark.parametrize("share", [0, 4])
+def test_a_request_that_breaks_down_leaves_its_batch_alone(share):
+    # Four requests in one context, one of them NaN, on all of the device and on
+    # a quarter of it (then a CTA's trees belong to one system after the other's).
+    # The others equal their solves alone, bit for bit.
+    d = domains.small(48, 16, 8, seed=7)
+    rhs = rhs_set(d, 3)
+    ref = solo(d, rhs)
+    bad = rhs[1].copy()
+    active = np.argwhere((d.flags & domains.ACTIVE) != 0)
+    bad[tuple(active[len(active) // 2])] = np.nan
+    srv = SolveServer(slots=1, batch=4)
+    try:
+        dom = srv.add_domain(d.flags, options(d, solve_share=share))
+        # Submitted during the set-up: all four wait when the driver starts.
+        reqs = [srv.submit(dom, bad if k == 1 else rhs[k]) for k in range(4)]
+        for k, req in enumerate(reqs):
+            st, res, x, _ = srv.poll(req, dom)
+            if k == 1:
+                assert st == 7, st  # HDD_ERR_BREAKDOWN
+                continue
+            assert st == 0 and res["iterations"] == ref[k][0], (k, st, res["iterations"])
+            assert np.array_equal(x, ref[k][1]), k
+    finally:
+        srv.close()
