@@ -453,7 +453,8 @@ void dispatch_cut(int nt, F f) {
 }
 template <class F>
 void dispatch_whole(int km, int nt, bool gs, F f) {
-    if (nt == 128) {  // trees of a few hundred unknowns at most: no slots
+    if (nt == 128) {  // small trees: slots in shared memory (ResidentSchedule::plan)
+        if (gs) throw Error(HDD_ERR_INTERNAL, "no kernel of four warps with slots in global memory");
         if (km == 1) f(Instance<1, 128, false>());
         else if (km == 2) f(Instance<2, 128, false>());
         else f(Instance<4, 128, false>());

@@ -608,9 +608,13 @@ bool ResidentSchedule::plan(const std::vector<ResidentPlan::Shape>& shapes,
         bare = std::max(bare, P.entries());
         all = std::max(all, P.entries() + P.slots);
     }
+    // CTAs of four warps keep their slots in shared memory (there is no kernel
+    // of theirs without): one tree's always fit, 8192 coefficients being at most
+    // as many unknowns and as many entries.
+    const int least = nt == 128 ? all : bare;
     km = 1;
     while (!cut && km < 4 && groups_for(km) > (size_t)nsm &&
-           ResidentPlan::smem_bytes(bare, 2 * km, nt) <= ResidentPlan::kMaxSmem)
+           ResidentPlan::smem_bytes(least, 2 * km, nt) <= ResidentPlan::kMaxSmem)
         km *= 2;
     global_slots = !cut && (ResidentPlan::smem_bytes(all, km, nt) > ResidentPlan::kMaxSmem || all >= 65536);
     entries = global_slots ? bare : all;

@@ -698,6 +698,56 @@ int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int
     }
 }
 
+// A forest of ntree trees of two fronts of one column each (child to parent
+// -0.5), the same for `members` factors of one class: its schedule, walked.
+// info as in shim_stream_walk; returns the largest error of the solution, which
+// is known in closed form, or -1 on an exception.
+double shim_forest_walk(int ntree, int members, int* info) {
+    try {
+        SnFactor F;
+        F.n = 2 * ntree;
+        for (int t = 0; t < ntree; ++t) {
+            F.perm.push_back(2 * t);
+            F.perm.push_back(2 * t + 1);
+            F.col0.push_back(2 * t);
+            F.col0.push_back(2 * t + 1);
+            F.ncol.insert(F.ncol.end(), {1, 1});
+            F.parent.insert(F.parent.end(), {2 * t + 1, -1});
+            F.rows.push_back({2 * t + 1});
+            F.rows.push_back({});
+            for (std::initializer_list<double> w : {std::initializer_list<double>{1.0, -0.5}, {1.0}}) {
+                F.Fw.emplace_back(w.size());
+                std::copy(w.begin(), w.end(), F.Fw.back().data());
+            }
+        }
+        std::vector<const SnFactor*> fs(members, &F);
+        std::vector<int> offs;
+        for (int m = 0; m < members; ++m) offs.push_back(m * F.n);
+        std::vector<ResidentPlan::Shape> shapes;
+        std::vector<std::vector<int>> mem;
+        whole_shapes(fs, offs, shapes, mem);
+        ResidentSchedule S;
+        if (!S.plan(shapes, mem, false, 148)) return -1.0;
+        std::vector<float> b((size_t)members * F.n), x(b.size(), 0.0f);
+        for (size_t i = 0; i < b.size(); ++i) b[i] = std::sin(0.37 * i);
+        std::vector<double> none;
+        StreamWalk W(S);
+        W.run(0, b.data(), x.data(), none, none, none);
+        const int v[10] = {1, S.km, S.nt, S.global_slots ? 1 : 0, (int)S.groups.size(), 0, (int)W.oob, (int)W.races,
+                           (int)W.ops, (int)W.barriers};
+        std::copy(v, v + 10, info);
+        double e = 0;
+        for (size_t i = 0; i < b.size(); i += 2) {
+            const double root = b[i + 1] - 0.5 * b[i];
+            e = std::max({e, std::fabs(x[i + 1] - root), std::fabs(x[i] - (b[i] - 0.5 * root))});
+            if (!(x[i] == x[i]) || !(x[i + 1] == x[i + 1])) return -1.0;
+        }
+        return e;
+    } catch (const std::exception&) {
+        return -1.0;
+    }
+}
+
 // Same plan: relative max-norm difference between its host solve (FP32
 // coefficients) and the factorisations' own FP64 solve, for a random
 // right-hand side; -1 on error.  *n gets the number of unknowns.

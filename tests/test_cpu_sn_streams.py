@@ -56,3 +56,17 @@ def test_schedules_read_nothing_but_their_own_system(name):
                 assert diff <= RTOL * float(np.max(np.abs(xe))), (level, kind, diff)
     finally:
         shim.shim_free(h)
+
+
+@pytest.mark.parametrize("trees,members", [(1, 1), (2700, 160), (2700, 320), (3400, 2)])
+def test_small_trees_keep_their_slots_in_shared_memory(trees, members):
+    # CTAs of four warps have no kernel with slots in global memory: thousands
+    # of tiny fronts, a few trees to a CTA, around the edge of shared memory and
+    # (3400) beyond four warps' coefficients.
+    shim = load_shim()
+    info = (C.c_int * 10)()
+    e = shim.shim_forest_walk(trees, members, info)
+    km, threads, in_memory = info[1], info[2], info[3]
+    assert 0 <= e <= 1.2e-7 and info[6] == 0 and info[7] == 0, (e, list(info))
+    assert threads == (128 if 3 * trees <= 8192 else 512)
+    assert not (threads == 128 and in_memory), (km, threads, in_memory)
