@@ -359,21 +359,9 @@ SigmaScratch SigmaGpu::primary() const {
     return sc;
 }
 
-int SigmaGpu::max_rhs() const {
-    int k = 4;
-    for (const SigmaLevel& L : lv) {
-        if (L.aii.nsn > 0) k = std::min(k, L.aii.kmax);
-        if (L.arr_solve.nsn > 0) k = std::min(k, L.arr_solve.kmax);
-    }
-    if (bottom.nsn > 0) k = std::min(k, bottom.kmax);
-    return k;
-}
-
 void SigmaGpu::alloc_scratch(SigmaScratch& sc, cudaStream_t s, int nrhs) const {
     free_scratch(sc);
     if (nrhs != 1 && nrhs != 2 && nrhs != 4) throw Error(HDD_ERR_INVALID_ARGUMENT, "systems per batch: 1, 2 or 4");
-    if (nrhs > max_rhs())
-        throw Error(HDD_ERR_UNSUPPORTED, "the interface solver's largest fronts leave no room for that many systems");
     size_t& b = sc.bytes;
     sc.nrhs = nrhs;
     sc.err = dev::alloc_zero<int>(1, b, s);

@@ -250,11 +250,9 @@ struct SolvePlan {
     bool whole_resident() const { return res.ngroups > 0 && !res.cut; }
     int n = 0;                       // total unknowns (concatenated)
     int nsn = 0, ntop = 0;           // fronts; those above the cut trees
-    int max_front = 0;               // of those
     int n_fwd = 0, n_tasks = 0;      // forward tasks, all tasks
     int ld_ctr = 0;                  // ints of one right-hand side's counters
     int grid = 0;                    // persistent CTAs of the task launch
-    int kmax = 1;                    // most right-hand sides one solve takes
     double solve_bytes = 0;          // algorithmic bytes of one solve, both directions
     int *d_rows = nullptr, *d_child = nullptr;
     int *d_gptr = nullptr, *d_gent = nullptr;  // gather lists (see sn_solve.cu)
@@ -381,8 +379,6 @@ struct SigmaGpu {
     void vcycle(const SigmaScratch& sc, bool u0_zero, cudaStream_t s, long long& launches, PhaseHook* hook = nullptr);
     SigmaScratch primary() const;
     void alloc_scratch(SigmaScratch& sc, cudaStream_t s, int nrhs = 1) const;
-    // Most right-hand sides every plan of this hierarchy takes in one launch.
-    int max_rhs() const;
     size_t scratch_bytes(int nrhs = 1) const;
     static void free_scratch(SigmaScratch& sc);
     // Nonzero when a bounded wait inside a supernodal solve gave up.

@@ -426,12 +426,6 @@ __global__ void __launch_bounds__(kNT, kPerSM) sn_task_kernel(PlanView P) {
 
 }  // namespace
 
-// Most unknowns a front above the trees may have rows and columns: each
-// right-hand side of a batch needs the vectors of the plan's largest front.
-size_t front_bytes(int max_front, int k) { return (size_t)(max_front + 4 * kNT) * k * sizeof(double); }
-constexpr size_t kSmemMax = 227 * 1024;
-constexpr size_t kFrontMax = 200 * 1024;
-
 void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s,
                       int* shared_err, double shrink) {
     release();
@@ -462,7 +456,6 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
     double total = 0;
     for (const SnFactor* F : factors) total += tree_weight(*F);
     if (shrink == 1 && resident_plan(factors, total) && res.build(factors, offsets, s)) {
-        kmax = 4;
         solve_bytes = res.solve_bytes;
         bytes = res.bytes;
         scratch();
@@ -493,7 +486,6 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
     std::vector<int> own;               // fronts whose coefficients are stored
     std::map<const SnFactor*, size_t> first_of;
     long long upd_total = 0, fw_total = 0;
-    max_front = 0;
     std::vector<int> rows, perm(n, 0);
     for (size_t f = 0; f < factors.size(); ++f) {
         const SnFactor& F = *factors[f];
@@ -520,7 +512,6 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
             } else {
                 T.fw = top[top_of[base[owner] + j]].fw;
             }
-            max_front = std::max(max_front, T.nj + nr);
             top_of[g] = (int)top.size();
             top.push_back(std::move(T));
         }
@@ -681,11 +672,6 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
         k.kids = T.kids.empty() ? 0 : 1;
     }
     stamp("gather lists");
-    if (front_bytes(max_front, 1) > kFrontMax)
-        throw Error(HDD_ERR_UNSUPPORTED, "supernodal front too large: " + std::to_string(max_front));
-    kmax = 1;
-    for (int k : {2, 4})
-        if (front_bytes(max_front, k) <= kSmemMax) kmax = k;
     std::vector<int> ntf, ntb;
     for (const Front& T : top) {
         ntf.push_back(T.ntf);
@@ -793,8 +779,8 @@ void SolvePlan::solve(const float* b_old, float* x_old, cudaStream_t s, long lon
 void SolvePlan::solve(const PlanScratch& sc, const float* b_old, float* x_old, cudaStream_t s, long long& launches,
                       PhaseHook* hook, int nrhs, long long ld_b, long long ld_x) const {
     if (nsn == 0) return;
-    if ((nrhs != 1 && nrhs != 2 && nrhs != 4) || nrhs > sc.nrhs || nrhs > kmax)
-        throw Error(HDD_ERR_INVALID_ARGUMENT, "right-hand sides per solve: 1, 2 or 4, within the scratch and the plan");
+    if ((nrhs != 1 && nrhs != 2 && nrhs != 4) || nrhs > sc.nrhs)
+        throw Error(HDD_ERR_INVALID_ARGUMENT, "right-hand sides per solve: 1, 2 or 4, within the scratch");
     if (hook) hook->begin(kPhaseSolve);
     const TopVectors top{sc.upd, sc.xnew, upd_len, (long long)std::max(n, 1), sc.ctr,
                          sc.ctr ? 1 + (long long)ld_ctr * nrhs : 0};

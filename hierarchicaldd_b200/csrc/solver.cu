@@ -360,13 +360,13 @@ void Solver::alloc_vectors(Work& w) {
 
 int Solver::max_batch() const {
     if (!initialized || opts.multilevel || L.global_vcycle) return 1;
-    return sigma.lv.empty() ? 4 : sigma.max_rhs();
+    return 4;
 }
 
 std::unique_ptr<Work> Solver::make_work(int k) {
     if (!initialized) throw Error(HDD_ERR_NOT_INITIALIZED, "initialize_preconditioner not called");
     if (k != 1 && k != 2 && k != 4) throw Error(HDD_ERR_INVALID_ARGUMENT, "systems per context: 1, 2 or 4");
-    if (k > max_batch()) throw Error(HDD_ERR_UNSUPPORTED, "the interface solver's fronts leave no room for that batch");
+    if (k > max_batch()) throw Error(HDD_ERR_UNSUPPORTED, "this domain's contexts hold one system");
     std::unique_ptr<Work> w(new Work());
     w->k = k;
     cuda_check(cudaSetDevice(opts.device), "cudaSetDevice");
@@ -1190,7 +1190,6 @@ void Solver::interface_solve_batch(int kind, int level, int nrhs, const float* b
     if (plan.nsn == 0 && rows > 0)
         throw Error(HDD_ERR_UNSUPPORTED, "no separate solve plan at this level (coarsest level solved as a whole)");
     if (rows == 0) return;
-    if (nrhs > plan.kmax) throw Error(HDD_ERR_UNSUPPORTED, "this plan's fronts leave no shared memory for that many right-hand sides");
     cuda_check(cudaSetDevice(opts.device), "cudaSetDevice");
     DevBuf<float> db, dx;
     db.upload(bh, (size_t)rows * nrhs, stream);

@@ -255,8 +255,8 @@ struct Solver {
     // Contexts run solves concurrently from different host threads; the
     // domain's own setup state is only read.
     std::unique_ptr<Work> make_work(int k = 1);
-    // Most systems a batch of this domain can hold (the interface solver's
-    // largest fronts bound it).
+    // Most systems a batch of this domain can hold: 4, or 1 with two-level DD or
+    // the whole-grid V-cycle.
     int max_batch() const;
     // Continuous batching: solves requests from the feeder on w's k systems
     // side by side until no system is busy and none is waiting.  A request

@@ -254,8 +254,7 @@ hdd_status hdd_interface_solve(hdd_solver* s, int kind, int level, const float* 
 /* Test seam: the same for nrhs (1, 2 or 4) right-hand sides at once, b and x
  * holding nrhs vectors of *n entries one after another.  The same
  * launches take all of them; each solution is bit-identical to
- * hdd_interface_solve of its right-hand side.  HDD_ERR_UNSUPPORTED when the
- * plan's largest front leaves no shared memory for nrhs vectors. */
+ * hdd_interface_solve of its right-hand side.  HDD_ERR_UNSUPPORTED as there. */
 hdd_status hdd_interface_solve_batch(hdd_solver* s, int kind, int level, int nrhs, const float* b, float* x, int* n);
 
 /* Interface DOF count at a sigma level and the level-0 DOF -> cell map

@@ -94,3 +94,29 @@ def test_every_route_matches_the_host_walk_and_its_batches(name):
     finally:
         s.close()
         shim.shim_free(h)
+
+
+def test_large_fronts_take_batches():
+    # A front of more than 6240 rows (140^3 of 8^3 subdomains: about 6500) is no
+    # reason to refuse right-hand sides side by side.
+    from hierarchicaldd_b200 import _lib
+    from hierarchicaldd_b200.solver import SPGrid_Domain_Decomposition_Solver
+    d = domains.small(140, 8, 5, seed=1)
+    m = d.meta
+    s = SPGrid_Domain_Decomposition_Solver()
+    lib = _lib.load()
+    try:
+        s.Set_Domain(d.flags, d.rhs)
+        s.Initialize_Preconditioner(m["vlevels"], d.size, d.sub_size, 2, m["nVcycles"], m["interior_smoothing"],
+                                    m["boundary_smoothing"], m["sigma_smoothing"], m["sigma_mg"])
+        nn = C.c_int()
+        assert lib.hdd_interface_solve(s.h, 0, 0, None, None, C.byref(nn)) == 0
+        rng = np.random.default_rng(5)
+        b = rng.uniform(-1, 1, (4, nn.value)).astype(np.float32)
+        x, xb = np.zeros_like(b), np.zeros_like(b)
+        for k in range(4):
+            assert lib.hdd_interface_solve(s.h, 0, 0, _fp(b[k]), _fp(x[k]), C.byref(nn)) == 0
+        assert lib.hdd_interface_solve_batch(s.h, 0, 0, 4, _fp(b), _fp(xb), C.byref(nn)) == 0, lib.hdd_last_error(s.h)
+        assert np.array_equal(xb, x)
+    finally:
+        s.close()
