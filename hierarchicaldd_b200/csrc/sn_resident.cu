@@ -244,7 +244,7 @@ __device__ __forceinline__ void op_product(Stream<D>& S, const Vec<K>& V, const 
             __syncwarp();
         }
         int c = h.y & 0xffff;
-        const int d = h.y >> 16;
+        const int d = (h.y >> 16) & 15;
         for (int g = 1; g < groups; ++g) {
             const int j[4] = {c, c + d, c + 2 * d, c + 3 * d};
             four_steps<K, D>(S, V.m, j, acc);
@@ -318,14 +318,15 @@ __device__ __forceinline__ void run_stream(Stream<D>& S, const Vec<K>& V) {
             if (count > 2 && l3.x >= 0) assemble_item<K, GS>(V, l3);
         } else if (type == kFinish) {
             const bool top = (h.x >> 8) & kTopRoot;
-            if (l1.x >= 0) finish_item<K, GS>(V, l1, h.y, h.z, top);
-            if (count > 1 && l2.x >= 0) finish_item<K, GS>(V, l2, h.y, h.z, top);
-            if (count > 2 && l3.x >= 0) finish_item<K, GS>(V, l3, h.y, h.z, top);
+            if (l1.x >= 0) finish_item<K, GS>(V, l1, h.y & 0xffff, h.z, top);
+            if (count > 1 && l2.x >= 0) finish_item<K, GS>(V, l2, h.y & 0xffff, h.z, top);
+            if (count > 2 && l3.x >= 0) finish_item<K, GS>(V, l3, h.y & 0xffff, h.z, top);
         } else if (type == kEnd) {
             return;
         }
-        if ((h.x >> 8) & kBar) __syncthreads();
-        else __syncwarp();
+        int bars = (int)((uint32_t)h.y >> 20);
+        if (bars == 0) __syncwarp();
+        for (; bars > 0; --bars) __syncthreads();
     }
 }
 

@@ -48,6 +48,7 @@ int groups_of(int rows, int cols) {
 // Index batches of a backward product after the header's two lines.
 int index_batches(int groups) { return groups <= 4 ? 0 : (groups - 4 + 7) / 8; }
 constexpr int kItems = 96;  // items of one assembly or finish
+constexpr int kMaxBars = 4095;
 
 }  // namespace
 
@@ -72,18 +73,15 @@ struct Block {
 void cut_level(const std::vector<Block>& blocks, bool fwd, ClassPlan& P, std::vector<std::vector<Op>>& out) {
     constexpr int kChunk = 128;
     const int nw = (int)out.size();
-    // Ends a phase: the warps' last operations carry the barrier.
-    std::vector<size_t> begun(nw);
-    for (int w = 0; w < nw; ++w) begun[w] = out[w].size();
+    // Ends a phase: a barrier more after the warps' last operations.
     auto barrier = [&]() {
-        for (int w = 0; w < nw; ++w) {
-            if (out[w].size() == begun[w]) {
+        for (auto& ops : out) {
+            if (ops.empty() || ops.back().bars == kMaxBars) {
                 Op b{};
                 b.type = kNothing;
-                out[w].push_back(b);
+                ops.push_back(b);
             }
-            out[w].back().flags |= kBar;
-            begun[w] = out[w].size();
+            ++ops.back().bars;
         }
     };
     auto col_range = [&](const Block& b, int r0, int rows, int& c0, int& c1) {
@@ -422,7 +420,7 @@ uint32_t* emit(const Op& o, const SnFactor& F, const ClassPlan& P, uint32_t* out
     auto header = [&](int lmq, int count, int a = 0, int b = 0) {
         for (int l = 0; l < 32; ++l) {
             h[4 * l] = o.type | lmq << 4 | o.flags << 8 | count << 16;
-            h[4 * l + 1] = a;
+            h[4 * l + 1] = a | (int)((uint32_t)o.bars << 20);
             h[4 * l + 2] = b;
         }
     };
@@ -466,7 +464,7 @@ uint32_t* emit(const Op& o, const SnFactor& F, const ClassPlan& P, uint32_t* out
     };
     if (!tr)
         for (int l = 0; l < 32; ++l) {
-            h[4 * l + 1] = (P.c0[i] + o.c0 + (l >> lmq)) | ns << 16;
+            h[4 * l + 1] |= (P.c0[i] + o.c0 + (l >> lmq)) | ns << 16;
             for (int u = 0; u < 4; ++u) h[4 * l + 2 + u / 2] |= input(l, 4 * (groups - 1) + u) << (u % 2 * 16);
         }
     auto rows_line = [&](int line, auto value) {  // one int per row, four a lane (the first slice's lanes)

@@ -39,16 +39,19 @@ HDD_HD constexpr int depth_of(int k) { return k == 1 ? 4 : 2; }
 
 // Operations of a stream.  Each starts with a batch whose first line is the
 // header, an int4 for every lane: {type | log2 of the lanes on row quads << 4 |
-// flags << 8 | count << 16, and three more words of the type}.
+// flags << 8 | count << 16, ... | CTA barriers after the operation << 20, two
+// words of the type}.  The barriers are a count, so that a warp without work in
+// a phase needs no operation for it.
 enum : int {
     kEnd = 0,
-    kNothing = 1,   // (a barrier)
+    kNothing = 1,   // barriers only
     // Items on 1 to 3 lines (count), one per lane: {index, first, second entry,
     // 1 when the index is a slot (GS)}: M[index] += the two entries.
     kAssemble = 2,
     // A block of a front times its inputs: count groups of four steps (a batch
     // each).  Header, forward: the lane's first column | distance to its next
-    // << 16, and the indices of the last group's four steps (16 bits each).
+    // << 16 (4 bits), and the indices of the last group's four steps (16 bits
+    // each).
     // Lines: destinations of four rows a lane; forward the rows' pairs of
     // children's entries (16 bits each) and one item of an assembly before
     // (index -1: none); backward the columns' indices for the first sixteen
@@ -58,14 +61,13 @@ enum : int {
     // written by another warp, and zero coefficients do not undo a NaN.
     kProduct = 3,
     // Items on 1 to 3 lines: {first partial sum, destination, first, second
-    // entry}.  Header: slices, distance between their partial sums.
+    // entry}.  Header: slices (16 bits), distance between their partial sums.
     kFinish = 4
 };
-constexpr int kBar = 1;        // CTA barrier after it
-constexpr int kPairs = 2;      // the rows have children's entries
-constexpr int kItem = 4;       // the product starts with an assembly
-constexpr int kTransposed = 8;
-constexpr int kTopRoot = 16;   // destinations -1 - entry are the plan above's update vectors
+constexpr int kPairs = 1;      // the rows have children's entries
+constexpr int kItem = 2;       // the product starts with an assembly
+constexpr int kTransposed = 4;
+constexpr int kTopRoot = 8;    // destinations -1 - entry are the plan above's update vectors
 // Indices are into the CTA's array M: the vector, rows outside cut trees, a
 // zero (a pair's missing entries), an unused entry (results of no row, never
 // read), partial sums and, where they fit, update slots.  GS: slots are in global memory
@@ -73,7 +75,7 @@ constexpr int kTopRoot = 16;   // destinations -1 - entry are the plan above's u
 
 // One operation of a warp, before it is written.
 struct Op {
-    int type, flags;
+    int type, flags, bars;            // bars: barriers after it
     int front, r0, rows, c0, c1, po;  // product; po: first of its partial sums (-1: not split)
     int i0, i1;                       // assembly, finish: items
     int nsl, stride;                  // finish

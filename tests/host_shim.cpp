@@ -136,7 +136,7 @@ struct StreamWalk {
                             for (;;) {
                                 if (pos[w] >= lim[w]) { ++oob; ++ended; break; }
                                 const long long h = pos[w];
-                                const int type = word(h, 0) & 15, flags = (word(h, 0) >> 8) & 255;
+                                const int type = word(h, 0) & 15;
                                 if (type == kEnd) {
                                     if (h + kBatch != lim[w]) ++oob;
                                     ++ended;
@@ -144,7 +144,8 @@ struct StreamWalk {
                                 }
                                 ++ops;
                                 pos[w] = operation(h, w, phase, M, at, slot, put, assemble);
-                                if (flags & kBar) { ++waiting; break; }
+                                owed[w] = (int)((uint32_t)word(h, 1) >> 20);
+                                if (owed[w] > 0) { --owed[w]; ++waiting; break; }
                             }
                         }
                         if (waiting > 0 && ended > 0) { ++oob; break; }  // warps at different barriers
@@ -173,7 +174,7 @@ struct StreamWalk {
                     if (!item(h + q, l, it)) continue;
                     if (type == kAssemble) { assemble(it, w, p); continue; }
                     double t = at(it[0], w, p);
-                    for (int s = 1; s < word(h, 1); ++s) t += at(it[0] + s * word(h, 2), w, p);
+                    for (int s = 1; s < (word(h, 1) & 0xffff); ++s) t += at(it[0] + s * word(h, 2), w, p);
                     put(it[1], (slot(it[2], w, p) + slot(it[3], w, p)) + t, flags, w, p);
                 }
             return h + kBatch;
@@ -198,7 +199,7 @@ struct StreamWalk {
                     int j;
                     if (tr) j = half(word(ix + (s0 + u) / 8, 4 * l + (s0 + u) % 8 / 2), u % 2);
                     else if (g + 1 == count) j = half(word(h, 4 * l + 2 + u / 2), u % 2);
-                    else j = half(word(h, 4 * l + 1), 0) + (4 * g + u) * half(word(h, 4 * l + 1), 1);
+                    else j = half(word(h, 4 * l + 1), 0) + (4 * g + u) * (half(word(h, 4 * l + 1), 1) & 15);
                     const double in = at(j, w, p);
                     for (int e = 0; e < 4; ++e)
                         acc[4 * l + e] = std::fma((double)words.at((size_t)(pos * (kLine / 4) + 4 * l + e)), in, acc[4 * l + e]);

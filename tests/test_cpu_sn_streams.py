@@ -18,6 +18,11 @@ from sn_routes import ROUTES, domain
 
 RTOL = 1.2e-7
 
+# Bytes of a domain's streams over those of the distinct coefficients they hold
+# (once per direction): the padding of small fronts, headers and indices.
+PADDING = {"one tree": 4.6, "pairs": 4.1, "quads": 3.7, "fronts in pairs": 3.7, "slots in memory": 3.2,
+           "cut factors": 3.4, "ragged": 4.5, "forest": 15.2}
+
 
 def _fp(a):
     return a.ctypes.data_as(C.POINTER(C.c_float))
@@ -39,6 +44,7 @@ def test_schedules_read_nothing_but_their_own_system(name):
                         flags.ctypes.data_as(C.POINTER(C.c_uint32)), err, 512)
     assert h, err.value
     rng = np.random.default_rng(3)
+    stream = coefficients = 0.0
     try:
         for level in range(levels):
             for kind in (0, 1):
@@ -54,6 +60,9 @@ def test_schedules_read_nothing_but_their_own_system(name):
                 assert np.all(np.isfinite(x)), (level, kind, "NaN from outside the system")
                 diff = float(np.max(np.abs(x.astype(np.float64) - xe)))
                 assert diff <= RTOL * float(np.max(np.abs(xe))), (level, kind, diff)
+                stream += by.value
+                coefficients += co.value
+        assert stream <= PADDING[name] * coefficients, stream / coefficients
     finally:
         shim.shim_free(h)
 
