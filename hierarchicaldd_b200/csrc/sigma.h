@@ -200,15 +200,16 @@ struct TopVectors {
 struct ResidentPlan {
     static constexpr size_t kMaxSmem = 226 * 1024;
     // Trees of one factor solved by one CTA: fronts first .. last (the root) of
-    // each; top: where the root's update vector goes in the plan above (-1: the
-    // root has none).  ext_off: index of the factor's unknown 0 in the solution
-    // of the plan above.
+    // each; top: where the root's update vector goes, from the first of the
+    // factor's update vectors in the plan above (-1: the root has none).
     struct Tree { int first, last, top; };
     struct Shape {
         const SnFactor* F = nullptr;
         std::vector<Tree> trees;
-        int ext_off = 0;
     };
+    // One use of a shape's factor: offset of its unknowns, and of its update
+    // vectors in the plan above.
+    struct Member { int off, top; };
     bool cut = false;                   // cut trees: separate forward and backward launches
     int n = 0, max_n = 0, ngroups = 0;  // unknowns; largest vector; CTAs of one solve (0: no plan)
     int km = 1, nt = 256;               // trees per CTA (1, 2 or 4), threads per CTA
@@ -228,8 +229,8 @@ struct ResidentPlan {
     // given the same SnFactor form a class that shares its coefficients.  False
     // when a CTA's shared memory does not hold the trees.
     bool build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s);
-    // Cut trees: shape i of the factor whose unknowns start at offsets[i].
-    bool build_cut(const std::vector<Shape>& shapes, const std::vector<int>& offsets, cudaStream_t s);
+    // Cut trees: shapes[i] for each of members[i].
+    bool build_cut(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members, cudaStream_t s);
     void release();
     // mode: 0 whole trees, both directions; 1 / 2 the forward / backward half of cut trees.
     void launch(int mode, const ResidentScratch& sc, const TopVectors& top, int* err, int grid_div,
@@ -239,7 +240,7 @@ struct ResidentPlan {
     void set_gate(int v, cudaStream_t s);
 
 private:
-    bool build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<int>>& members, cudaStream_t s);
+    bool build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members, cudaStream_t s);
 };
 
 // Device plan for a batch of independent supernodal triangular solves.

@@ -57,7 +57,7 @@ struct RView {
     const RWarp* warps;
     const int* off;                    // member -> first unknown
     const int* perm;
-    const int* ext;                    // cut trees: unknowns of the plan above
+    const int* ext;                    // cut trees: unknowns of the plan above, from the member's first
     const char* stream;
     double *upd, *y;
     double* top_upd;                   // cut trees: the plan above's update vectors and solution
@@ -360,7 +360,7 @@ __device__ __forceinline__ void solve_group(const RView& P, const RGroup& G, int
     Vec<K> V;
     V.m = reinterpret_cast<double*>(smem + (size_t)(NT / 32) * D * kBatchBytes);
     V.upd = P.upd + rhs * P.ld_upd + G.upd;
-    V.top = P.top_upd + rhs * P.ld_top_upd;
+    V.top = P.top_upd + rhs * P.ld_top_upd + G.top;
     double* y = P.y + rhs * P.ld_y + G.y;
     Stream<D> S;
     S.start(P.stream + G.stream + (long long)(W.first + (MODE == kBackward ? W.nf : 0)) * kLine,
@@ -390,7 +390,7 @@ __device__ __forceinline__ void solve_group(const RView& P, const RGroup& G, int
     if (MODE == kBackward) {
         const double* tx = P.top_x + rhs * P.ld_top_x;
         for (int i = threadIdx.x; i < G.n; i += NT) V.m[i] = y[i];
-        for (int i = threadIdx.x; i < G.next; i += NT) V.m[G.n + i] = tx[P.ext[G.ext + i]];
+        for (int i = threadIdx.x; i < G.next; i += NT) V.m[G.n + i] = tx[off[0] + P.ext[G.ext + i]];
         __syncthreads();
     }
     if (MODE != kForward) {
@@ -476,22 +476,21 @@ void dispatch_whole(int km, int nt, bool gs, F f) {
 bool ResidentPlan::build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s) {
     release();
     std::vector<Shape> shapes;
-    std::vector<std::vector<int>> members;
+    std::vector<std::vector<Member>> members;
     whole_shapes(factors, offsets, shapes, members);
     for (size_t f = 0; f < factors.size(); ++f) n = std::max(n, offsets[f] + factors[f]->n);
     cut = false;
     return build_shapes(shapes, members, s);
 }
 
-bool ResidentPlan::build_cut(const std::vector<Shape>& shapes, const std::vector<int>& offsets, cudaStream_t s) {
+bool ResidentPlan::build_cut(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members,
+                             cudaStream_t s) {
     release();
-    std::vector<std::vector<int>> members;
-    for (int o : offsets) members.push_back({o});
     cut = true;
     return build_shapes(shapes, members, s);
 }
 
-bool ResidentPlan::build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<int>>& members,
+bool ResidentPlan::build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members,
                                 cudaStream_t s) {
     int dev_id = 0, nsm = 0;
     dev::ck(cudaGetDevice(&dev_id), "cudaGetDevice");

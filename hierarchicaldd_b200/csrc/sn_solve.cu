@@ -465,15 +465,30 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
     }
     // The lower trees of every factor go to one CTA each (sn_resident.cu); the
     // tasks below are those of the fronts above them.
-    std::vector<char> low(nsn, 0), cut_root(nsn, 0);
+    // Members given the same factor share its trees' streams and the coefficients
+    // of its fronts above.
+    std::map<const SnFactor*, FactorCut> cuts;
+    for (const SnFactor* F : factors) cuts.emplace(F, FactorCut());
+    {
+        std::vector<std::pair<const SnFactor* const, FactorCut>*> each;
+        for (auto& c : cuts) each.push_back(&c);
+        const double cap = cut_weight(total) / shrink;
+        std::string failed;
+#pragma omp parallel for schedule(dynamic)
+        for (size_t i = 0; i < each.size(); ++i) {
+            try {
+                each[i]->second = cut_trees(*each[i]->first, cap);
+            } catch (const std::exception& e) {
+#pragma omp critical
+                failed = e.what();
+            }
+        }
+        if (!failed.empty()) throw Error(HDD_ERR_UNSUPPORTED, failed);
+    }
     std::vector<ResidentPlan::Shape> shapes;
-    std::vector<int> shape_off;
-    std::vector<std::vector<int>> shape_roots;  // plan fronts of the trees' roots
-    const double cap = cut_weight(total) / shrink;
-    for (size_t f = 0; f < factors.size(); ++f)
-        cut_trees(*factors[f], offsets[f], base[f], cap, low, cut_root, shapes, shape_off, shape_roots);
-    // The fronts above, numbered in post-order, factor by factor.  Members given
-    // the same factor share its coefficients.
+    std::vector<std::vector<ResidentPlan::Member>> members;
+    std::map<const SnFactor*, size_t> shape0;  // a factor's first shape
+    // The fronts above, numbered in post-order, factor by factor.
     struct Front {
         int f, j, nj, nr, col0, parent, height, depth, upd;
         long long fw, rows_off, gp, ge;
@@ -490,16 +505,21 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
     for (size_t f = 0; f < factors.size(); ++f) {
         const SnFactor& F = *factors[f];
         const size_t owner = first_of.emplace(&F, f).first->second;
+        const FactorCut& C = cuts.at(&F);
+        if (owner == f) {
+            shape0[&F] = shapes.size();
+            shapes.insert(shapes.end(), C.shapes.begin(), C.shapes.end());
+            members.resize(shapes.size());
+        }
+        if (upd_total + C.upd_len >= (long long)INT32_MAX)
+            throw Error(HDD_ERR_UNSUPPORTED, "update vectors too large for 32-bit indices");
+        for (size_t i = 0; i < C.shapes.size(); ++i)
+            members[shape0[&F] + i].push_back({offsets[f], (int)upd_total});
         for (int i = 0; i < F.n; ++i) perm[offsets[f] + i] = offsets[f] + F.perm[i];
         for (int j = 0; j < (int)F.col0.size(); ++j) {
             const int g = base[f] + j, nr = (int)F.rows[j].size();
-            if (!low[g] || cut_root[g]) {
-                if (upd_total + nr >= (long long)INT32_MAX)
-                    throw Error(HDD_ERR_UNSUPPORTED, "update vectors too large for 32-bit indices");
-                upd_off[g] = (int)upd_total;
-                upd_total += nr;
-            }
-            if (low[g]) continue;
+            if (C.upd[j] >= 0) upd_off[g] = (int)upd_total + C.upd[j];
+            if (C.low[j]) continue;
             Front T{};
             T.f = (int)f; T.j = j; T.nj = F.ncol[j]; T.nr = nr; T.col0 = offsets[f] + F.col0[j]; T.upd = upd_off[g];
             T.rows_off = (long long)rows.size();
@@ -520,13 +540,9 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
             if (top_of[g] >= 0) top[top_of[g]].parent = p >= 0 ? top_of[base[f] + p] : -1;
             if (p >= 0 && top_of[base[f] + p] >= 0) top[top_of[base[f] + p]].kids.push_back(g);
         }
+        upd_total += C.upd_len;
     }
-    for (size_t i = 0; i < shapes.size(); ++i)
-        for (size_t t = 0; t < shapes[i].trees.size(); ++t) {
-            ResidentPlan::Tree& tree = shapes[i].trees[t];
-            if (!shapes[i].F->rows[tree.last].empty()) tree.top = upd_off[shape_roots[i][t]];
-        }
-    if (!shapes.empty() && !res.build_cut(shapes, shape_off, s)) {
+    if (!shapes.empty() && !res.build_cut(shapes, members, s)) {
         // Trees with unusually many update entries: smaller ones, in the end none.
         build(factors, offsets, s, shared_err, shrink * 4);
         return;

@@ -263,7 +263,7 @@ void plan_class(const ResidentPlan::Shape& T, int nwarps, ClassPlan& P) {
     }
     for (const auto& t : T.trees) {
         ext_base.push_back(P.n + (int)P.ext.size());
-        for (int r : F.rows[t.last]) P.ext.push_back(T.ext_off + r);
+        for (int r : F.rows[t.last]) P.ext.push_back(r);
     }
     const int ns = (int)P.fronts.size();
     P.zero = P.n + (int)P.ext.size();
@@ -534,7 +534,7 @@ size_t ResidentPlan::smem_bytes(int entries, int k, int nt) {
 }
 
 void whole_shapes(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets,
-                  std::vector<ResidentPlan::Shape>& shapes, std::vector<std::vector<int>>& members) {
+                  std::vector<ResidentPlan::Shape>& shapes, std::vector<std::vector<ResidentPlan::Member>>& members) {
     std::map<const SnFactor*, int> shape_of;
     for (size_t f = 0; f < factors.size(); ++f) {
         const SnFactor* F = factors[f];
@@ -552,12 +552,12 @@ void whole_shapes(const std::vector<const SnFactor*>& factors, const std::vector
             shapes.push_back(std::move(T));
             members.emplace_back();
         }
-        members[it->second].push_back(offsets[f]);
+        members[it->second].push_back({offsets[f], 0});
     }
 }
 
 bool ResidentSchedule::plan(const std::vector<ResidentPlan::Shape>& shapes,
-                            const std::vector<std::vector<int>>& members, bool cut_trees, int nsm) {
+                            const std::vector<std::vector<ResidentPlan::Member>>& members, bool cut_trees, int nsm) {
     cut = cut_trees;
     shape = &shapes;
     double biggest = 0;
@@ -577,13 +577,13 @@ bool ResidentSchedule::plan(const std::vector<ResidentPlan::Shape>& shapes,
     }
     // Sixteen warps, or four where a tree is a few lines a warp; cut trees that
     // are more than the SMs run two CTAs to an SM.
-    if (cut) nt = shapes.size() > (size_t)nsm ? 256 : 512;
-    else nt = biggest <= 8192 ? 128 : 512;
     auto groups_for = [&](int k) {
         size_t g = 0;
         for (const auto& m : members) g += (m.size() + k - 1) / k;
         return g;
     };
+    if (cut) nt = groups_for(1) > (size_t)nsm ? 256 : 512;
+    else nt = biggest <= 8192 ? 128 : 512;
     cp.assign(shapes.size(), ClassPlan());
     std::vector<std::string> err(shapes.size());
 #pragma omp parallel for schedule(dynamic)
@@ -666,7 +666,8 @@ bool ResidentSchedule::plan(const std::vector<ResidentPlan::Shape>& shapes,
                 if (cut) y_len += cp[c].n;
                 const int kk = cnt > 1 ? km : 1;
                 if (global_slots) upd_len += (long long)kk * ((cp[c].slots + 2) & ~1);
-                for (int i = 0; i < cnt; ++i) off.push_back(members[c][m + i]);
+                G.top = members[c][m].top;
+                for (int i = 0; i < cnt; ++i) off.push_back(members[c][m + i].off);
                 groups.push_back(G);
             }
     upd_len = std::max<long long>(upd_len, 2);
@@ -707,10 +708,11 @@ bool resident_plan(const std::vector<const SnFactor*>& factors, double total) {
     return largest <= kCutCost + total / kCutRate;
 }
 
-void cut_trees(const SnFactor& F, int off, int base, double cap, std::vector<char>& low, std::vector<char>& cut_root,
-               std::vector<ResidentPlan::Shape>& shapes, std::vector<int>& shape_off,
-               std::vector<std::vector<int>>& shape_roots) {
+FactorCut cut_trees(const SnFactor& F, double cap) {
     const int ns = (int)F.col0.size();
+    FactorCut C;
+    C.low.assign(ns, 0);
+    C.upd.assign(ns, -1);
     std::vector<double> weight(ns);
     std::vector<int> size(ns, 1), len(ns);
     for (int j = 0; j < ns; ++j) {
@@ -725,26 +727,33 @@ void cut_trees(const SnFactor& F, int off, int base, double cap, std::vector<cha
     auto fits = [&](int j) { return weight[j] <= cap && (len[j] + (int)F.rows[j].size()) <= kCutLen; };
     double w = 0;
     int n = 0;
+    std::vector<char> root(ns, 0);
     for (int j = 0; j < ns; ++j) {
         if (!fits(j) || (F.parent[j] >= 0 && fits(F.parent[j]))) continue;
         const int vec = len[j] + (int)F.rows[j].size();
-        if (shape_off.empty() || shapes.back().F != &F || shape_off.back() != off || w + weight[j] > cap ||
-            n + vec > kCutLen) {
-            shapes.emplace_back();
-            shapes.back().F = &F;
-            shapes.back().ext_off = off;
-            shape_off.push_back(off);
-            shape_roots.emplace_back();
+        if (C.shapes.empty() || w + weight[j] > cap || n + vec > kCutLen) {
+            C.shapes.emplace_back();
+            C.shapes.back().F = &F;
             w = 0;
             n = 0;
         }
         w += weight[j];
         n += vec;
-        shapes.back().trees.push_back({j - size[j] + 1, j, -1});
-        shape_roots.back().push_back(base + j);
-        cut_root[base + j] = 1;
-        for (int i = j - size[j] + 1; i <= j; ++i) low[base + i] = 1;
+        C.shapes.back().trees.push_back({j - size[j] + 1, j, -1});
+        root[j] = 1;
+        for (int i = j - size[j] + 1; i <= j; ++i) C.low[i] = 1;
     }
+    for (int j = 0; j < ns; ++j) {
+        if (C.low[j] && !root[j]) continue;
+        if (C.upd_len >= (long long)INT32_MAX)
+            throw Error(HDD_ERR_UNSUPPORTED, "update vectors too large for 32-bit indices");
+        C.upd[j] = (int)C.upd_len;
+        C.upd_len += (long long)F.rows[j].size();
+    }
+    for (ResidentPlan::Shape& S : C.shapes)
+        for (ResidentPlan::Tree& T : S.trees)
+            if (!F.rows[T.last].empty()) T.top = C.upd[T.last];
+    return C;
 }
 
 }  // namespace hdd

@@ -28,7 +28,8 @@ struct RGroup {
     int n, perm;              // unknowns; offset of perm
     int next, ext;            // unknowns of the plan above that cut trees read; offset of their indices
     int warps;                // offset of the class's warps
-    int member0, count, pad;
+    int member0, count;
+    int top;                  // cut trees: the member's first update vector in the plan above
 };
 
 constexpr int kLine = 512;              // bytes of a line: 16 a lane
@@ -113,11 +114,10 @@ struct ResidentSchedule {
     std::vector<int> off, perm, ext;
     long long upd_len = 0, y_len = 0;    // doubles of the scratch
     double coef = 0;                     // coefficients of one direction, each class's once
-    // Schedules shapes[c] for members[c] (offsets of their unknowns) on a device
-    // of nsm SMs; false when a CTA's shared memory does not hold the trees.
+    // Schedules shapes[c] for members[c] on a device of nsm SMs; false when a CTA's shared memory does not hold the trees.
     // The shapes are referred to until the streams are written.
-    bool plan(const std::vector<ResidentPlan::Shape>& shapes, const std::vector<std::vector<int>>& members, bool cut_trees,
-              int nsm);
+    bool plan(const std::vector<ResidentPlan::Shape>& shapes,
+              const std::vector<std::vector<ResidentPlan::Member>>& members, bool cut_trees, int nsm);
     // The streams, one per class and warp, in floats: `total` in all (padding
     // that prefetches run into included), stream i from at(i) on.
     size_t streams() const { return stream.size(); }
@@ -134,7 +134,7 @@ private:
 
 // Whole factors: a shape per distinct factor, and its members' offsets.
 void whole_shapes(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets,
-                  std::vector<ResidentPlan::Shape>& shapes, std::vector<std::vector<int>>& members);
+                  std::vector<ResidentPlan::Shape>& shapes, std::vector<std::vector<ResidentPlan::Member>>& members);
 
 // What a factor's trees weigh for the rules below.
 double tree_weight(const SnFactor& F);
@@ -143,11 +143,16 @@ double tree_weight(const SnFactor& F);
 bool resident_plan(const std::vector<const SnFactor*>& factors, double total);
 // The heaviest tree cut from a plan of weight `total`.
 double cut_weight(double total);
-// The lower trees of factor F (unknowns from `off` on, fronts from `base` on in
-// the plan): the largest subtrees of at most weight `cap`, each marked in low /
-// cut_root; consecutive ones share a CTA up to that weight.
-void cut_trees(const SnFactor& F, int off, int base, double cap, std::vector<char>& low, std::vector<char>& cut_root,
-               std::vector<ResidentPlan::Shape>& shapes, std::vector<int>& shape_off,
-               std::vector<std::vector<int>>& shape_roots);
+// The lower trees of factor F: the largest subtrees of at most weight `cap`;
+// consecutive ones share a CTA (a shape) up to that weight.
+struct FactorCut {
+    std::vector<char> low;            // fronts of the trees
+    std::vector<ResidentPlan::Shape> shapes;
+    // Offsets of the update vectors of the trees' roots and the fronts above
+    // (-1: of the others), and their length in all.
+    std::vector<int> upd;
+    long long upd_len = 0;
+};
+FactorCut cut_trees(const SnFactor& F, double cap);
 
 }  // namespace hdd

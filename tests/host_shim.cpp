@@ -8,6 +8,7 @@
 #include <exception>
 #include <functional>
 #include <limits>
+#include <map>
 #include <random>
 #include <string>
 #include <vector>
@@ -99,8 +100,8 @@ struct StreamWalk {
                     } else if (S.global_slots) {
                         if (d == -1) ++oob;  // the zero slot
                         U.write(-1 - d, v, w, p);
-                    } else if ((flags & kTopRoot) && mode == 1 && -1 - d < (int)top_upd.size()) {
-                        top_upd[-1 - d] = v;
+                    } else if ((flags & kTopRoot) && mode == 1 && G.top - 1 - d < (int)top_upd.size()) {
+                        top_upd[G.top - 1 - d] = v;
                     } else {
                         ++oob;
                     }
@@ -116,7 +117,7 @@ struct StreamWalk {
                 for (int i = 0; i < G.n; ++i)
                     M.write(i, mode == 2 ? y.at(G.y + i) : (double)b[off + S.perm.at(G.perm + i)], -1, phase);
                 if (mode == 2)
-                    for (int i = 0; i < G.next; ++i) M.write(G.n + i, top_x.at(S.ext.at(G.ext + i)), -1, phase);
+                    for (int i = 0; i < G.next; ++i) M.write(G.n + i, top_x.at(off + S.ext.at(G.ext + i)), -1, phase);
                 for (int pass = mode == 2 ? 1 : 0; pass < (mode == 1 ? 1 : 2); ++pass) {
                     ++phase;
                     std::vector<long long> pos(nw), lim(nw);
@@ -587,7 +588,8 @@ int shim_plan_emulate(void* h, int kind, int level, const float* b, float* x) {
 // trees, or the lower trees of every factor with the fronts above them solved
 // front by front.  info: {1 whole / 0 cut, trees per CTA, threads per CTA, 1 when
 // update slots are in global memory, CTAs, fronts above, accesses out of range,
-// races between warps, operations, barriers}; *bytes: of the streams, *coef: the
+// races between warps, operations, barriers, streams of trees (members with the
+// same factor share one)}; *bytes: of the streams, *coef: the
 // distinct coefficients' of both directions.  Returns 0, or 1 on an exception.
 int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int* info, double* bytes, double* coef) {
     try {
@@ -600,7 +602,7 @@ int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int
         double total = 0;
         for (const SnFactor* F : fs) total += tree_weight(*F);
         std::vector<ResidentPlan::Shape> shapes;
-        std::vector<std::vector<int>> members;
+        std::vector<std::vector<ResidentPlan::Member>> members;
         std::vector<double> y, upd, sol;
         ResidentSchedule S;
         constexpr int kSMs = 148;
@@ -612,9 +614,9 @@ int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int
         int ntop = 0;
         std::vector<long long> counts(4, 0);
         auto done = [&](const StreamWalk& W) {
-            const int v[10] = {whole ? 1 : 0, S.km, S.nt, S.global_slots ? 1 : 0, (int)S.groups.size(), ntop,
-                               (int)W.oob, (int)W.races, (int)W.ops, (int)W.barriers};
-            std::copy(v, v + 10, info);
+            const int v[11] = {whole ? 1 : 0, S.km, S.nt, S.global_slots ? 1 : 0, (int)S.groups.size(), ntop,
+                               (int)W.oob, (int)W.races, (int)W.ops, (int)W.barriers, (int)shapes.size()};
+            std::copy(v, v + 11, info);
             *bytes = 4.0 * S.total();
             *coef = 8.0 * S.coef;
         };
@@ -624,24 +626,23 @@ int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int
             done(W);
             return 0;
         }
-        std::vector<int> base(fs.size() + 1, 0), shape_off;
-        for (size_t f = 0; f < fs.size(); ++f) base[f + 1] = base[f] + (int)fs[f]->col0.size();
-        std::vector<char> low(base.back(), 0), root(base.back(), 0);
-        std::vector<std::vector<int>> roots;
-        for (size_t f = 0; f < fs.size(); ++f)
-            cut_trees(*fs[f], offs[f], base[f], cut_weight(total), low, root, shapes, shape_off, roots);
-        // Update vectors of the fronts above and of the trees' roots.
-        std::vector<int> at(base.back(), -1);
-        for (size_t f = 0; f < fs.size(); ++f)
-            for (size_t j = 0; j < fs[f]->col0.size(); ++j)
-                if (!low[base[f] + j] || root[base[f] + j]) {
-                    at[base[f] + j] = (int)upd.size();
-                    upd.resize(upd.size() + fs[f]->rows[j].size(), std::numeric_limits<double>::quiet_NaN());
-                }
-        for (size_t i = 0; i < shapes.size(); ++i)
-            for (size_t t = 0; t < shapes[i].trees.size(); ++t)
-                if (!shapes[i].F->rows[shapes[i].trees[t].last].empty()) shapes[i].trees[t].top = at[roots[i][t]];
-        for (int o : shape_off) members.push_back({o});
+        // Update vectors of the fronts above and of the trees' roots, factor by factor.
+        std::map<const SnFactor*, FactorCut> cuts;
+        std::map<const SnFactor*, size_t> shape0;
+        std::vector<long long> first;
+        for (size_t f = 0; f < fs.size(); ++f) {
+            const auto c = cuts.emplace(fs[f], FactorCut());
+            FactorCut& C = c.first->second;
+            if (c.second) {
+                C = cut_trees(*fs[f], cut_weight(total));
+                shape0[fs[f]] = shapes.size();
+                shapes.insert(shapes.end(), C.shapes.begin(), C.shapes.end());
+                members.resize(shapes.size());
+            }
+            first.push_back((long long)upd.size());
+            for (size_t i = 0; i < C.shapes.size(); ++i) members[shape0[fs[f]] + i].push_back({offs[f], (int)upd.size()});
+            upd.resize(upd.size() + (size_t)C.upd_len, std::numeric_limits<double>::quiet_NaN());
+        }
         S = ResidentSchedule();
         if (!S.plan(shapes, members, true, kSMs)) return 1;
         StreamWalk W(S);
@@ -652,13 +653,14 @@ int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int
         sol.assign(n, 0.0);
         for (size_t f = 0; f < fs.size(); ++f) {
             const SnFactor& F = *fs[f];
+            const FactorCut& C = cuts.at(fs[f]);
             const int ns = (int)F.col0.size();
             std::vector<std::vector<int>> kids(ns);
             for (int j = 0; j < ns; ++j)
                 if (F.parent[j] >= 0) kids[F.parent[j]].push_back(j);
             std::vector<std::vector<double>> yv(ns);
             for (int j = 0; j < ns; ++j) {
-                if (low[base[f] + j]) continue;
+                if (C.low[j]) continue;
                 ++ntop;
                 const int nj = F.ncol[j], nr = (int)F.rows[j].size(), m = nj + nr;
                 std::vector<double> v(m, 0.0);
@@ -669,17 +671,17 @@ int shim_stream_walk(void* h, int kind, int level, const float* b, float* x, int
                         const int i = r < F.col0[j] + nj ? r - F.col0[j]
                                                          : nj + (int)(std::lower_bound(F.rows[j].begin(), F.rows[j].end(), r) -
                                                                       F.rows[j].begin());
-                        v[i] += upd[at[base[f] + c] + q];
+                        v[i] += upd.at(first[f] + C.upd[c] + q);
                     }
                 for (int r = 0; r < m; ++r) {
                     double s = 0;
                     for (int c = 0; c < nj; ++c) s += (double)(float)F.Fw[j][(size_t)c * m + r] * v[c];
                     if (r < nj) yv[j].push_back(s);
-                    else upd[at[base[f] + j] + r - nj] = v[r] + s;
+                    else upd.at(first[f] + C.upd[j] + r - nj) = v[r] + s;
                 }
             }
             for (int j = ns - 1; j >= 0; --j) {
-                if (low[base[f] + j]) continue;
+                if (C.low[j]) continue;
                 const int nj = F.ncol[j], m = nj + (int)F.rows[j].size();
                 for (int a = 0; a < nj; ++a) {
                     double s = 0;
@@ -725,7 +727,7 @@ double shim_forest_walk(int ntree, int members, int* info) {
         std::vector<int> offs;
         for (int m = 0; m < members; ++m) offs.push_back(m * F.n);
         std::vector<ResidentPlan::Shape> shapes;
-        std::vector<std::vector<int>> mem;
+        std::vector<std::vector<ResidentPlan::Member>> mem;
         whole_shapes(fs, offs, shapes, mem);
         ResidentSchedule S;
         if (!S.plan(shapes, mem, false, 148)) return -1.0;

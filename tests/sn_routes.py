@@ -2,7 +2,8 @@
 the CPU and GPU tests of those."""
 from hierarchicaldd_b200 import domains
 
-ROUTES = ["one tree", "pairs", "quads", "fronts in pairs", "slots in memory", "cut factors", "ragged", "forest"]
+ROUTES = ["one tree", "pairs", "quads", "fronts in pairs", "slots in memory", "cut factors",
+          "equal cut factors", "ragged", "forest"]
 
 
 def domain(name):
@@ -17,8 +18,10 @@ def domain(name):
         return domains.small(96, 16, 20, seed=4), 3
     if name == "slots in memory":       # 32^3 interiors: update slots do not fit
         return domains.small(128, 32, 24, seed=4), 2
-    if name == "cut factors":           # few large trees: cut, members sharing coefficients
+    if name == "cut factors":           # few large trees: cut
         return domains.small(64, 32, 9, seed=4), 2
+    if name == "equal cut factors":     # ... most of them with the same factor
+        return domains.small((96, 64, 64), 32, 0, seed=4), 2
     if name == "ragged":
         return domains.small((33, 40, 41), 16, 5, seed=4), 2
     # Many components: plans of thousands of tiny fronts, trees without fronts above.

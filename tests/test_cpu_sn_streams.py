@@ -21,7 +21,7 @@ RTOL = 1.2e-7
 # Bytes of a domain's streams over those of the distinct coefficients they hold
 # (once per direction): the padding of small fronts, headers and indices.
 PADDING = {"one tree": 4.6, "pairs": 4.1, "quads": 3.7, "fronts in pairs": 3.7, "slots in memory": 3.2,
-           "cut factors": 3.4, "ragged": 4.5, "forest": 15.2}
+           "cut factors": 3.4, "equal cut factors": 3.9, "ragged": 4.5, "forest": 15.2}
 
 
 def _fp(a):
@@ -53,13 +53,15 @@ def test_schedules_read_nothing_but_their_own_system(name):
                     continue
                 b = rng.uniform(-1, 1, n).astype(np.float32)
                 x, xe = np.full(n, np.nan, np.float32), np.zeros(n, np.float32)
-                info, by, co = (C.c_int * 10)(), C.c_double(), C.c_double()
+                info, by, co = (C.c_int * 11)(), C.c_double(), C.c_double()
                 assert shim.shim_stream_walk(h, kind, level, _fp(b), _fp(x), info, C.byref(by), C.byref(co)) == 0
                 assert shim.shim_plan_emulate(h, kind, level, _fp(b), _fp(xe)) == 0
                 assert info[6] == 0 and info[7] == 0, (level, kind, "out of range, races", info[6], info[7])
                 assert np.all(np.isfinite(x)), (level, kind, "NaN from outside the system")
                 diff = float(np.max(np.abs(x.astype(np.float64) - xe)))
                 assert diff <= RTOL * float(np.max(np.abs(xe))), (level, kind, diff)
+                if name == "equal cut factors" and kind == 1 and level == 0:
+                    assert info[0] == 0 and 2 * info[10] <= info[4], list(info)
                 stream += by.value
                 coefficients += co.value
         assert stream <= PADDING[name] * coefficients, stream / coefficients
