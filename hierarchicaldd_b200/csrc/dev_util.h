@@ -39,65 +39,90 @@ T* alloc_zero(size_t n, size_t& bytes, cudaStream_t s) {
     return p;
 }
 
+// Two pinned buffers through which a setup's plans go to the device in turn.
+// Pinning and unpinning 64 MB takes about as long as copying it several times
+// over, so one pair serves all plans of a setup and grows as they need it.
+class Staging {
+public:
+    Staging() = default;
+    Staging(const Staging&) = delete;
+    Staging& operator=(const Staging&) = delete;
+    ~Staging() {
+        free_buffers();
+        for (cudaEvent_t e : copied_)
+            if (e) cudaEventDestroy(e);
+    }
+    void reserve(size_t floats) {
+        for (cudaEvent_t& e : copied_)
+            if (!e) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+        if (floats <= size_) return;
+        free_buffers();
+        for (float*& b : buf_) ck(cudaMallocHost(&b, floats * sizeof(float)), "pinned staging");
+        size_ = floats;
+    }
+    size_t size() const { return size_; }
+    // The next buffer, once its last copy has been made.
+    float* next() {
+        at_ ^= 1;
+        ck(cudaEventSynchronize(copied_[at_]), "staging reuse");
+        return buf_[at_];
+    }
+    // Copies the buffer next() gave.
+    void copy(float* dst, size_t floats, cudaStream_t s) {
+        if (floats > 0)
+            ck(cudaMemcpyAsync(dst, buf_[at_], floats * sizeof(float), cudaMemcpyHostToDevice, s), "coefficient upload");
+        ck(cudaEventRecord(copied_[at_], s), "event");
+    }
+
+private:
+    void free_buffers() {
+        for (cudaEvent_t e : copied_)
+            if (e) cudaEventSynchronize(e);
+        for (float*& b : buf_) {
+            if (b) cudaFreeHost(b);
+            b = nullptr;
+        }
+        size_ = 0;
+    }
+    float* buf_[2] = {nullptr, nullptr};
+    cudaEvent_t copied_[2] = {nullptr, nullptr};
+    size_t size_ = 0;
+    int at_ = 0;
+};
+
 // A device array of `total` floats made of n items, item i at at(i) (ascending;
-// it ends where the next begins) and written by pack(i, dst) in parallel.  The
-// items go through two pinned staging buffers in turn, each copied to the device
-// while the next is packed: the gigabytes of a large solve plan then cross at
-// pinned-copy speed and the packing overlaps the copy.  Returns once the
-// staging buffers are free again.
+// it ends where the next begins) and written by pack(i, dst) in parallel: one
+// staging buffer is copied while the next is packed.
 template <class At, class Pack>
-void upload_packed(size_t n, long long total, At at, Pack pack, cudaStream_t s, float*& d, size_t& bytes) {
+void upload_packed(size_t n, long long total, At at, Pack pack, Staging& stage, cudaStream_t s, float*& d, size_t& bytes) {
     const long long alloc = std::max<long long>(total, 4);
     d = nullptr;
     if (cudaMalloc(&d, (size_t)alloc * sizeof(float)) != cudaSuccess)
         throw Error(HDD_ERR_OUT_OF_MEMORY, "cudaMalloc: supernodal coefficients");
-    auto end_of = [&](size_t i) { return i + 1 < n ? (long long)at(i + 1) : total; };
-    long long biggest = 4;
-    for (size_t i = 0; i < n; ++i) biggest = std::max(biggest, end_of(i) - (long long)at(i));
-    // Floats per staging buffer: 32 MB (pinning costs about as much as the
-    // copy, so the buffers stay small), or the largest item.
-    const long long chunk = std::max<long long>(biggest, 8ll << 20);
-    float* stage[2] = {nullptr, nullptr};
-    cudaEvent_t copied[2] = {nullptr, nullptr};
-    auto cleanup = [&]() {
-        for (int i = 0; i < 2; ++i) {
-            if (copied[i]) { cudaEventSynchronize(copied[i]); cudaEventDestroy(copied[i]); }
-            if (stage[i]) cudaFreeHost(stage[i]);
-        }
-    };
     try {
-        for (int i = 0; i < 2; ++i) {
-            ck(cudaMallocHost(&stage[i], (size_t)std::min(chunk, alloc) * sizeof(float)), "pinned staging");
-            ck(cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming), "event");
-        }
-        size_t g0 = 0;
-        int buf = 0;
-        bool used[2] = {false, false};
-        while (g0 < n) {
+        auto end_of = [&](size_t i) { return i + 1 < n ? (long long)at(i + 1) : total; };
+        long long biggest = 4;
+        for (size_t i = 0; i < n; ++i) biggest = std::max(biggest, end_of(i) - (long long)at(i));
+        // Floats per chunk: 16 MB, or the largest item.
+        const long long chunk = std::max<long long>(biggest, 4ll << 20);
+        stage.reserve((size_t)std::min(chunk, alloc));
+        for (size_t g0 = 0, g1; g0 < n; g0 = g1) {
             // Items g0 .. g1-1 fill this chunk (at least one item).
             const long long base = at(g0);
-            size_t g1 = g0 + 1;
-            while (g1 < n && end_of(g1) - base <= chunk) ++g1;
-            const long long end = end_of(g1 - 1);
-            if (used[buf]) ck(cudaEventSynchronize(copied[buf]), "staging reuse");
-            float* st = stage[buf];
+            for (g1 = g0 + 1; g1 < n && end_of(g1) - base <= chunk; ++g1) {}
+            float* st = stage.next();
 #pragma omp parallel for schedule(dynamic)
             for (size_t g = g0; g < g1; ++g) pack(g, st + ((long long)at(g) - base));
-            if (end > base)
-                ck(cudaMemcpyAsync(d + base, st, (size_t)(end - base) * sizeof(float), cudaMemcpyHostToDevice, s),
-                   "coefficient upload");
-            ck(cudaEventRecord(copied[buf], s), "event");
-            used[buf] = true;
-            buf ^= 1;
-            g0 = g1;
+            stage.copy(d + base, (size_t)(end_of(g1 - 1) - base), s);
         }
         if (total < alloc)  // an empty plan's placeholder
             ck(cudaMemsetAsync(d + total, 0, (size_t)(alloc - total) * sizeof(float), s), "memset");
     } catch (...) {
-        cleanup();
+        cudaStreamSynchronize(s);
+        cudaFree(d);
+        d = nullptr;
         throw;
     }
-    cleanup();
     bytes += (size_t)alloc * sizeof(float);
 }
 

@@ -155,6 +155,7 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
     };
     M = ih.M;
     smoothing = smoothing_iterations;
+    dev::Staging stage;
     {
         size_t b0 = 0;
         d_err = dev::alloc_zero<int>(1, b0, s);
@@ -223,8 +224,8 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
             std::vector<int> offs;
             for (int sd = 0; sd < ih.n_sub; ++sd)
                 if (ih.Aii[l][sd].rows > 0) { fs.push_back(&aii[rep[sd]]); offs.push_back(off[sd]); }
-            L.aii.build(fs, offs, s, d_err);
-            L.arr_solve.build({&arrf}, {0}, s, d_err);
+            L.aii.build(fs, offs, stage, s, d_err);
+            L.arr_solve.build({&arrf}, {0}, stage, s, d_err);
             device_bytes += L.aii.bytes + L.arr_solve.bytes;
             stamp("device plans", l);
         } else {
@@ -282,8 +283,8 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
                 std::vector<int> offs;
                 for (int sd = 0; sd < ih.n_sub; ++sd)
                     if (ih.Aii[l][sd].rows > 0) { fs.push_back(&aii[rep[sd]]); offs.push_back(off[sd]); }
-                L.aii.build(fs, offs, s, d_err);
-                L.arr_solve.build({&arrf}, {0}, s, d_err);
+                L.aii.build(fs, offs, stage, s, d_err);
+                L.arr_solve.build({&arrf}, {0}, stage, s, d_err);
                 device_bytes += L.aii.bytes + L.arr_solve.bytes;
                 stamp("device plans (coarsest level, literal smoothing)", l);
                 continue;
@@ -326,7 +327,7 @@ void SigmaGpu::setup(const InterfaceHost& ih, int smoothing_iterations, cudaStre
             kf.analyze(K, have_xyz ? &kxyz : nullptr);
             kf.factor(K, eps);
             kf.build_solve_blocks();
-            bottom.build({&kf}, {0}, s, d_err);
+            bottom.build({&kf}, {0}, stage, s, d_err);
             n_bottom = nb;
             n_bottom_int = ni;
             size_t b2 = 0;

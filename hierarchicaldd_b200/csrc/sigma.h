@@ -18,6 +18,7 @@
 namespace hdd {
 
 struct DomainLayout;
+namespace dev { class Staging; }
 
 struct CsrF {
     int rows = 0, cols = 0;
@@ -228,9 +229,11 @@ struct ResidentPlan {
     // Whole factors: factors[i] solves the unknowns from offsets[i] on; members
     // given the same SnFactor form a class that shares its coefficients.  False
     // when a CTA's shared memory does not hold the trees.
-    bool build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s);
+    bool build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, dev::Staging& stage,
+               cudaStream_t s);
     // Cut trees: shapes[i] for each of members[i].
-    bool build_cut(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members, cudaStream_t s);
+    bool build_cut(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members, dev::Staging& stage,
+                   cudaStream_t s);
     void release();
     // mode: 0 whole trees, both directions; 1 / 2 the forward / backward half of cut trees.
     void launch(int mode, const ResidentScratch& sc, const TopVectors& top, int* err, int grid_div,
@@ -240,7 +243,8 @@ struct ResidentPlan {
     void set_gate(int v, cudaStream_t s);
 
 private:
-    bool build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members, cudaStream_t s);
+    bool build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members,
+                      dev::Staging& stage, cudaStream_t s);
 };
 
 // Device plan for a batch of independent supernodal triangular solves.
@@ -274,8 +278,8 @@ struct SolvePlan {
     size_t bytes = 0;
     // shared_err: an error word shared with other plans (owned by the caller),
     // or null for a word of the plan's own.  shrink: divides the size of cut trees.
-    void build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s,
-               int* shared_err = nullptr, double shrink = 1);
+    void build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, dev::Staging& stage,
+               cudaStream_t s, int* shared_err = nullptr, double shrink = 1);
     void release();
     long long part_len = 0, upd_len = 0;  // doubles in a scratch's partial-sum and update buffers
     // x_old = (A+eps I)^{-1} b_old (both in the concatenated original order),

@@ -473,25 +473,26 @@ void dispatch_whole(int km, int nt, bool gs, F f) {
 
 }  // namespace
 
-bool ResidentPlan::build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s) {
+bool ResidentPlan::build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, dev::Staging& stage,
+                         cudaStream_t s) {
     release();
     std::vector<Shape> shapes;
     std::vector<std::vector<Member>> members;
     whole_shapes(factors, offsets, shapes, members);
     for (size_t f = 0; f < factors.size(); ++f) n = std::max(n, offsets[f] + factors[f]->n);
     cut = false;
-    return build_shapes(shapes, members, s);
+    return build_shapes(shapes, members, stage, s);
 }
 
 bool ResidentPlan::build_cut(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members,
-                             cudaStream_t s) {
+                             dev::Staging& stage, cudaStream_t s) {
     release();
     cut = true;
-    return build_shapes(shapes, members, s);
+    return build_shapes(shapes, members, stage, s);
 }
 
 bool ResidentPlan::build_shapes(const std::vector<Shape>& shapes, const std::vector<std::vector<Member>>& members,
-                                cudaStream_t s) {
+                                dev::Staging& stage, cudaStream_t s) {
     int dev_id = 0, nsm = 0;
     dev::ck(cudaGetDevice(&dev_id), "cudaGetDevice");
     dev::ck(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev_id), "SM count");
@@ -511,7 +512,7 @@ bool ResidentPlan::build_shapes(const std::vector<Shape>& shapes, const std::vec
     bytes = 0;
     float* d = nullptr;
     dev::upload_packed(S.streams(), S.total(), [&](size_t i) { return S.at(i); },
-                       [&](size_t i, float* dst) { S.write(i, dst); }, s, d, bytes);
+                       [&](size_t i, float* dst) { S.write(i, dst); }, stage, s, d, bytes);
     d_stream = reinterpret_cast<char*>(d);
     auto nonempty = [](std::vector<int>& v) -> const std::vector<int>& {
         if (v.empty()) v.push_back(0);

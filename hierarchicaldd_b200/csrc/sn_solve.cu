@@ -426,8 +426,8 @@ __global__ void __launch_bounds__(kNT, kPerSM) sn_task_kernel(PlanView P) {
 
 }  // namespace
 
-void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, cudaStream_t s,
-                      int* shared_err, double shrink) {
+void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::vector<int>& offsets, dev::Staging& stage,
+                      cudaStream_t s, int* shared_err, double shrink) {
     release();
     const bool verbose = std::getenv("HDD_VERBOSE") != nullptr;
     const auto t_start = std::chrono::steady_clock::now();
@@ -455,7 +455,7 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
     if (nsn == 0) return;
     double total = 0;
     for (const SnFactor* F : factors) total += tree_weight(*F);
-    if (shrink == 1 && resident_plan(factors, total) && res.build(factors, offsets, s)) {
+    if (shrink == 1 && resident_plan(factors, total) && res.build(factors, offsets, stage, s)) {
         solve_bytes = res.solve_bytes;
         bytes = res.bytes;
         scratch();
@@ -542,9 +542,9 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
         }
         upd_total += C.upd_len;
     }
-    if (!shapes.empty() && !res.build_cut(shapes, members, s)) {
+    if (!shapes.empty() && !res.build_cut(shapes, members, stage, s)) {
         // Trees with unusually many update entries: smaller ones, in the end none.
-        build(factors, offsets, s, shared_err, shrink * 4);
+        build(factors, offsets, stage, s, shared_err, shrink * 4);
         return;
     }
     stamp("trees uploaded");
@@ -626,7 +626,7 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
                                for (int r = m; r < ld; ++r) dst[(size_t)c * ld + r] = 0.0f;
                            }
                        },
-                       s, d_fw, bytes);
+                       stage, s, d_fw, bytes);
     stamp("coefficients packed and uploaded");
     // Gather lists: the children's update entries per position of a front, in
     // child order; and the children it waits for.
