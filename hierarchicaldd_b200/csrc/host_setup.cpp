@@ -397,4 +397,46 @@ void dense_to_pages(const int size[3], long long n, const int32_t* origin, const
     for_page_cells(size, n, origin, [&](size_t e, size_t d) { values[e] = dense[d]; });
 }
 
+// Both: the dense staging buffer (4 B per grid cell), six PCG vectors plus flags
+// over the stored tiles (26 B per tile cell, 8 B more for the FP64 iterate of
+// the precision form) and the V-cycle level flags (about 1.2 B per tile cell).
+// The interface solver (matrices, solve plans, vectors) holds between 183 B
+// (256^3, sub 32) and 1290 B per Active cell: the streams of small plans and of
+// sparse domains' tiny fronts are mostly padding.  Measured, MB and stored tiles:
+// sub 8: 3.6 and 8, 46 and 150, 149 and 512 (214 with the exact coarse solve), 623
+// and 1728 (942); sub 16: 24 and 8, 62 and 26 (bubble), 115 and 80, 326 and 216
+// (exact), 1576 and 1000; sub 32: 129 and 8, 161 and 27, 629 and 64 (exact), 1461
+// and 216, 3072 and 512, sparse 150 and 56; two-level, sub 64: 306 and 2.  An
+// exact solve of the coarsest level grows with how fine that level is: 128^3, sub
+// 32, with 3, 2 and 1 sigma levels 442 (629 with more spheres), 1042 and 6954;
+// 96^3, sub 16: 296, 552 and 2630.
+DeviceEstimate estimate_device_bytes(const hdd_options& o, const uint32_t* flags) {
+    const long long n0 = o.size[0], n1 = o.size[1], n2 = o.size[2];
+    const int s = std::max(1, o.sub_size[0]);
+    const long long t0 = (n0 + s - 1) / s, t1 = (n1 + s - 1) / s, t2 = (n2 + s - 1) / s;
+    std::vector<uint8_t> used((size_t)(t0 * t1 * t2), 0);
+    long long active = 0;
+    for (long long i = 0; i < n0; ++i)
+        for (long long j = 0; j < n1; ++j)
+            for (long long k = 0; k < n2; ++k)
+                if (flags[(i * n1 + j) * n2 + k] & F_ACTIVE) {
+                    ++active;
+                    used[(size_t)(((i / s) * t1 + j / s) * t2 + k / s)] = 1;
+                }
+    long long tiles = 0;
+    for (uint8_t u : used) tiles += u;
+    const long long tile_cells = tiles * s * s * s;
+    const long long vectors =
+        4 * n0 * n1 * n2 + (o.precision_mode == HDD_PRECISION_MIXED ? 36 : 28) * tile_cells + (16ll << 20);
+    long long interface = 700 * tile_cells, per_active = 1400;
+    if (s <= 8) interface = 800 * tile_cells + (4ll << 20);
+    else if (s <= 16) interface = 420 * tile_cells + (36ll << 20);
+    else if (s <= 32) interface = 220 * tile_cells + (84ll << 20);
+    if (o.coarse_solve == HDD_COARSE_EXACT) {
+        interface = o.sigma_levels >= 3 ? interface * 27 / 20 : (o.sigma_levels == 2 ? 2 : 16) * interface;
+        if (o.sigma_levels < 2) per_active = 4000;
+    }
+    return {vectors + 56 * active, vectors + std::min(interface, per_active * active)};
+}
+
 }  // namespace hdd

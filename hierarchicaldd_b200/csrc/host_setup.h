@@ -129,4 +129,11 @@ void flag_faces(const int n[3], uint32_t* f);
 void flag_boundary(const int n[3], uint32_t* f);
 void number_of_subdomains(const int size[3], const int sub[3], int out[3]);
 
+// Device bytes of a domain, known before its setup: what it cannot do without,
+// and what it holds at most.
+struct DeviceEstimate {
+    long long least, most;
+};
+DeviceEstimate estimate_device_bytes(const hdd_options& o, const uint32_t* flags);
+
 }  // namespace hdd

@@ -18,8 +18,9 @@
 // on different domains.  Every system of every context runs the same kernels
 // in the same order, so a request's result does not depend on which context,
 // which batch or how many others ran beside it.
-// Domains are admitted in arrival order once their estimated device footprint
-// fits the HBM budget; their host setup (layout, interface assembly,
+// Domains are admitted in arrival order once the upper estimate of their device
+// footprint fits the HBM budget (one that may not fit is admitted alone, one
+// that cannot is refused); their host setup (layout, interface assembly,
 // factorisation) runs on a worker with setup_threads OpenMP threads, so
 // setups overlap with solves of other domains.
 #include <omp.h>
@@ -37,6 +38,7 @@
 #include <thread>
 #include <vector>
 
+#include "host_setup.h"
 #include "solver.h"
 
 using hdd::Error;
@@ -80,32 +82,6 @@ struct Request {
     std::vector<float> x;
     Clock::time_point t_submit, t_done;
 };
-
-// Device footprint estimate made before the setup: the dense staging buffer
-// (4 B per grid cell), six PCG vectors plus flags over the stored tiles
-// (26 B per tile cell, 8 B more for the FP64 iterate of the precision form),
-// the V-cycle level flags (about 1.2 B per tile cell) and the interface
-// solver's factors and FP64 vectors (56 B per Active cell, an upper estimate
-// from the 64^3..256^3 sphere domains).
-long long estimate_bytes(const hdd_options& o, const uint32_t* flags) {
-    const long long n0 = o.size[0], n1 = o.size[1], n2 = o.size[2];
-    const int s = std::max(1, o.sub_size[0]);
-    const long long t1 = (n1 + s - 1) / s, t2 = (n2 + s - 1) / s, t0 = (n0 + s - 1) / s;
-    std::vector<uint8_t> used((size_t)(t0 * t1 * t2), 0);
-    long long active = 0;
-    for (long long i = 0; i < n0; ++i)
-        for (long long j = 0; j < n1; ++j)
-            for (long long k = 0; k < n2; ++k)
-                if (flags[(i * n1 + j) * n2 + k] & 0x10000u) {
-                    ++active;
-                    used[(size_t)(((i / s) * t1 + j / s) * t2 + k / s)] = 1;
-                }
-    long long tiles = 0;
-    for (uint8_t u : used) tiles += u;
-    const long long tile_cells = tiles * s * s * s;
-    const long long per_tile_cell = o.precision_mode == HDD_PRECISION_MIXED ? 36 : 28;
-    return 4 * n0 * n1 * n2 + per_tile_cell * tile_cells + 56 * active + (16ll << 20);
-}
 
 }  // namespace
 
@@ -202,6 +178,7 @@ struct hdd_server {
             }
             for (int i = 0; i < 3; ++i) dd.ctx_bytes[i] = (long long)dd.solver->work_bytes(1 << i);
             dd.state = DomainState::Resident;
+            admit();  // it may hold less than it was admitted for
         } else {
             reserved -= dd.reserved;
             dd.reserved = 0;
@@ -472,9 +449,10 @@ hdd_status hdd_server_add_domain(hdd_server* srv, const hdd_options* opts, const
         d.opts.device = srv->opt.device;
         const size_t n = (size_t)opts->size[0] * opts->size[1] * opts->size[2];
         d.flags.assign(flags, flags + n);
-        d.reserved = estimate_bytes(d.opts, flags);
+        const hdd::DeviceEstimate e = hdd::estimate_device_bytes(d.opts, flags);
+        d.reserved = e.most;
         std::lock_guard<std::mutex> lk(srv->mu);
-        if (d.reserved > srv->budget) return HDD_ERR_OUT_OF_MEMORY;
+        if (e.least > srv->budget) return HDD_ERR_OUT_OF_MEMORY;
         const long long id = srv->next_id++;
         srv->domains.emplace(id, std::move(d));
         srv->admission.push_back(id);

@@ -319,8 +319,9 @@ void hdd_destroy(hdd_solver* s);
  * No counterpart in the reference, whose GPU demo solves one domain per
  * process (GPU/Test_Bench_3D/main.cpp) through one worker thread per GPU
  * (GPU/Nodes/Command.h:33-55).  A server owns `slots` worker threads.  A domain
- * added with hdd_server_add_domain is admitted, in arrival order, once its
- * estimated device footprint fits the HBM budget; a worker then runs its setup
+ * added with hdd_server_add_domain is admitted, in arrival order, once the upper
+ * estimate of its device footprint fits the HBM budget (or alone, when nothing
+ * else holds memory); a worker then runs its setup
  * (as hdd_initialize_preconditioner) and the domain stays resident until
  * removed.  Each solve request names a resident (or still setting-up) domain
  * and a right-hand side.  A resident domain keeps a pool of solve contexts (the
@@ -346,8 +347,8 @@ void hdd_server_options_default(hdd_server_options* opts);
 hdd_status hdd_server_create(const hdd_server_options* opts, hdd_server** out);
 
 /* Queues a domain for setup (flags are copied; opts as for hdd_create, its
- * device ignored).  Returns at once; HDD_ERR_OUT_OF_MEMORY when the domain's
- * estimated footprint alone exceeds the budget. */
+ * device ignored).  Returns at once; HDD_ERR_OUT_OF_MEMORY when the least the
+ * domain takes exceeds the budget. */
 hdd_status hdd_server_add_domain(hdd_server* srv, const hdd_options* opts, const uint32_t* flags,
                                  long long* domain_id);
 
@@ -372,7 +373,7 @@ hdd_status hdd_server_poll(hdd_server* srv, long long request_id, int wait_ms, h
  * its budget. */
 hdd_status hdd_server_remove_domain(hdd_server* srv, long long domain_id);
 
-/* Device bytes held by admitted domains (estimates until set up, then what
+/* Device bytes held by admitted domains (upper estimates until set up, then what
  * their solvers and solve contexts hold) and the budget. */
 hdd_status hdd_server_memory(hdd_server* srv, long long* reserved, long long* budget);
 

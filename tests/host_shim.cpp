@@ -751,6 +751,13 @@ double shim_forest_walk(int ntree, int members, int* info) {
     }
 }
 
+// A server's estimates of a domain's device bytes, {least, most}.
+void shim_estimate(const hdd_options* o, const uint32_t* flags, long long* bytes) {
+    const DeviceEstimate e = estimate_device_bytes(*o, flags);
+    bytes[0] = e.least;
+    bytes[1] = e.most;
+}
+
 // Same plan: relative max-norm difference between its host solve (FP32
 // coefficients) and the factorisations' own FP64 solve, for a random
 // right-hand side; -1 on error.  *n gets the number of unknowns.

@@ -57,6 +57,7 @@ def load_shim():
     L.shim_plan_check.restype = C.c_double
     L.shim_plan_check.argtypes = [C.c_void_p, C.c_int, C.c_int, ip]
     L.shim_plan_emulate.argtypes = [C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_float)]
+    L.shim_estimate.argtypes = [C.c_void_p, C.POINTER(C.c_uint32), C.POINTER(C.c_longlong)]
     L.shim_forest_walk.restype = C.c_double
     L.shim_forest_walk.argtypes = [C.c_int, C.c_int, ip]
     L.shim_stream_walk.argtypes = [C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_float), C.POINTER(C.c_float), ip,

@@ -255,3 +255,64 @@ def test_a_request_that_breaks_down_leaves_its_batch_alone(share):
             assert np.array_equal(x, ref[k][1]), k
     finally:
         srv.close()
+
+
+def test_the_budget_covers_domains_in_setup():
+    # What a domain holds is at most what it was admitted for: two domains of
+    # which the budget holds one never have more than the budget reserved.
+    d = domains.small(64, 16, 12, seed=7)
+    probe = SolveServer(slots=1)
+    try:
+        probe.wait_domain(probe.add_domain(d.flags, options(d)))
+        holds = probe.memory()[0]
+    finally:
+        probe.close()
+    srv = SolveServer(slots=2, hbm_budget_bytes=int(holds * 1.9))
+    try:
+        ids = [srv.add_domain(d.flags, options(d)) for _ in range(2)]
+        reqs = [srv.submit(dom, d.rhs) for dom in ids]
+        most = 0
+        for dom, req in zip(ids, reqs):
+            if dom == ids[0]:  # both set up, if both were admitted
+                srv.wait_domain(ids[0])
+                srv.wait_domain(ids[1], wait_ms=1500)
+            while True:
+                most = max(most, srv.memory()[0])
+                r = srv.poll(req, dom, wait_ms=1, want_x=False)
+                if r is not None:
+                    break
+            assert r[0] == 0
+            most = max(most, srv.memory()[0])
+            srv.remove_domain(dom)
+        assert most <= srv.memory()[1], (most, srv.memory()[1], holds)
+    finally:
+        srv.close()
+
+
+@pytest.mark.parametrize("name,extra", [("16", {}), ("40", {}), ("48", {}), ("64", {}), ("96", {"coarse_solve": 1}),
+                                        ("96", {"precision_mode": 1}), ("bubble", {}), ("union", {}), ("flat", {})])
+def test_the_estimate_covers_what_a_domain_holds(name, extra):
+    import ctypes as C
+    from shim_ffi import load_shim
+    if name == "bubble":
+        d = domains.reference_generator((49, 49, 49), (4, 24, 24))
+        d = domains.Domain(d.size, d.flags, d.rhs, (16, 16, 16), d.name, dict(domains.small(48, 16, 8).meta))
+    elif name == "union":
+        d = domains.config5(16)
+        d = domains.Domain(d.size, d.flags, d.rhs, (16, 16, 16), d.name, dict(domains.small(48, 16, 8).meta))
+    else:
+        d = {"16": lambda: domains.small(16, 8, 3), "40": lambda: domains.small((40, 36, 44), 8, 6),
+             "48": lambda: domains.small(48, 16, 8), "64": lambda: domains.small(64, 32, 8),
+             "96": lambda: domains.small(96, 16, 20), "flat": lambda: domains.small((16, 72, 90), 8, 3)}[name]()
+    o = options(d, **extra)
+    est = (C.c_longlong * 2)()
+    flags = np.ascontiguousarray(d.flags, np.uint32)
+    load_shim().shim_estimate(C.byref(o), flags.ctypes.data_as(C.POINTER(C.c_uint32)), est)
+    srv = SolveServer(slots=1)
+    try:
+        dom = srv.add_domain(d.flags, o)
+        assert srv.wait_domain(dom)
+        holds = srv.memory()[0]
+        assert holds <= est[1] and est[0] <= est[1], (holds, est[0], est[1])
+    finally:
+        srv.close()
