@@ -28,6 +28,20 @@ def _fp(a):
     return a.ctypes.data_as(C.POINTER(C.c_float))
 
 
+# Interface solves of each domain that take the route it is named for: (kind, level)
+# and {field of the walk's info: value}; whole 0, trees per CTA 1, threads 2,
+# slots in global memory 3, CTAs 4, fronts above the cut 5.
+TAKES = {"one tree": {(0, 0): {0: 1, 4: 1}},
+         "pairs": {(1, 0): {0: 1, 1: 2, 2: 128}, (0, 0): {0: 0, 2: 512}},
+         "quads": {(1, 0): {0: 1, 1: 4, 2: 128}, (0, 0): {0: 0, 2: 256}},
+         "fronts in pairs": {(1, 0): {0: 1, 1: 2, 2: 512, 3: 0}, (0, 0): {0: 0}},
+         "slots in memory": {(1, 0): {0: 1, 1: 1, 2: 512, 3: 1}},
+         "cut factors": {(1, 0): {0: 0}},
+         "equal cut factors": {(1, 0): {0: 0}},
+         "ragged": {(1, 0): {0: 1, 1: 1}, (0, 0): {0: 0}},
+         "forest": {(0, 1): {0: 0, 5: 0}, (1, 0): {0: 1, 1: 4}}}
+
+
 def _unknowns(shim, h, kind, level):
     shape = (C.c_int * 3)()
     subs = range(shim.shim_num_subdomains(h)) if kind else [0]
@@ -60,6 +74,8 @@ def test_schedules_read_nothing_but_their_own_system(name):
                 assert np.all(np.isfinite(x)), (level, kind, "NaN from outside the system")
                 diff = float(np.max(np.abs(x.astype(np.float64) - xe)))
                 assert diff <= RTOL * float(np.max(np.abs(xe))), (level, kind, diff)
+                for i, v in TAKES[name].get((kind, level), {}).items():
+                    assert info[i] == v, (name, kind, level, list(info))
                 if name == "equal cut factors" and kind == 1 and level == 0:
                     assert info[0] == 0 and 2 * info[10] <= info[4], list(info)
                 stream += by.value

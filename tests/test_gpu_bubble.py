@@ -69,3 +69,30 @@ def test_bubble_domain(size, sub, delta, multilevel):
         assert np.linalg.norm(x - xo) / np.linalg.norm(xo) < 1e-5
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("vlevels,interior,boundary", [(1, 3, 3), (2, 3, 3), (2, 2, 1), (2, 0, 0)])
+def test_whole_grid_vcycle_with_a_large_bottom_level(vlevels, interior, boundary):
+    # A bottom level of more than 23^3 cells does not fit one CTA: its sweeps are
+    # launches that change between two copies of u.
+    d = domains.reference_generator((65, 65, 65), (8, 32, 32))
+    m = dict(META, vlevels=vlevels, interior_smoothing=interior, boundary_smoothing=boundary)
+    from hierarchicaldd_b200.solver import SPGrid_Domain_Decomposition_Solver
+    s = SPGrid_Domain_Decomposition_Solver()
+    s.Set_Domain(d.flags, d.rhs)
+    s.Initialize_Preconditioner(vlevels, d.size, (16,) * 3, 2, 1, interior, boundary, 3, 1)
+    o = Oracle(d.size, (16,) * 3, d.flags, **m)
+    try:
+        f0 = o.level_flags(0)
+        rng = np.random.default_rng(22)
+        u = rng.standard_normal(d.size).astype(np.float32)
+        u[(f0 & (ACTIVE | INTERFACE)) == 0] = 0
+        b = rng.standard_normal(d.size).astype(np.float32)
+        b[(f0 & ACTIVE) == 0] = 0
+        uo, r = u.copy(), np.zeros_like(u)
+        for nv in (1, 2):
+            ug = s.V_Cycle(u, b, nv)
+            uo, r = o.vcycle(uo, r, b)
+            assert np.array_equal(ug, uo), (nv, np.max(np.abs(ug - uo)))
+    finally:
+        s.close()

@@ -172,26 +172,32 @@ def test_pcg_config1_against_fp64_oracle():
     assert err7 <= 1e-5, err7
 
 
-@pytest.mark.parametrize("cluster", ["1", "2"])
-def test_vcycle_sub16_cluster_variants_bitexact(cluster, monkeypatch):
-    """The 16^3 V-cycle runs either in one CTA or split over a 2-CTA cluster."""
-    monkeypatch.setenv("HDD_VCYCLE_CLUSTER", cluster)
-    d = domains.small(48, 16, 8, seed=7)
-    s, o = make_pair(d)
+@pytest.mark.parametrize("sub,n,levels", [(8, 24, (1, 2, 3)), (16, 48, (1, 2, 3, 4)), (32, 64, (1, 2, 3, 4, 5))])
+def test_vcycle_of_every_depth_bitexact(sub, n, levels):
+    """Every number of levels of a box, from the bottom's sweeps alone to a
+    coarsest level of one cell, one and two V-cycles, with smoothing counts that
+    end on either copy of u, and none."""
+    d = domains.small(n, sub, n // 6, seed=7)
     rng = np.random.default_rng(8)
-    f0 = o.level_flags(0)
-    u = rng.standard_normal(d.size).astype(np.float32)
-    u[(f0 & (ACTIVE | INTERFACE)) == 0] = 0
-    b = rng.standard_normal(d.size).astype(np.float32)
-    b[(f0 & ACTIVE) == 0] = 0
-    ug = s.V_Cycle(u, b, 1)
-    s.close()
-    uo, _ = o.vcycle(u, np.zeros_like(u), b)
-    assert np.array_equal(ug, uo), np.max(np.abs(ug - uo))
+    for vlevels in levels:
+        for interior, boundary in ((3, 3), (2, 1), (0, 0)):
+            d.meta.update(vlevels=vlevels, interior_smoothing=interior, boundary_smoothing=boundary)
+            s, o = make_pair(d)
+            f0 = o.level_flags(0)
+            u = rng.standard_normal(d.size).astype(np.float32)
+            u[(f0 & (ACTIVE | INTERFACE)) == 0] = 0
+            b = rng.standard_normal(d.size).astype(np.float32)
+            b[(f0 & ACTIVE) == 0] = 0
+            uo, r = u.copy(), np.zeros_like(u)
+            for nv in (1, 2):
+                ug = s.V_Cycle(u, b, nv)
+                uo, r = o.vcycle(uo, r, b)
+                assert np.array_equal(ug, uo), (vlevels, interior, boundary, nv, np.max(np.abs(ug - uo)))
+            s.close()
 
 
-def test_sub32_cluster_vcycle_and_pcg():
-    """32^3 subdomains use the 4-CTA cluster kernel: bit-exact V-cycle, PCG parity."""
+def test_sub32_vcycle_and_pcg():
+    """32^3 subdomains (vcycle_kernel_32): bit-exact V-cycle, PCG parity."""
     d = domains.small(64, 32, 10, seed=9)
     d.meta.update(vlevels=4, interior_smoothing=4, boundary_smoothing=4, sigma_levels=4)
     s, o = make_pair(d)

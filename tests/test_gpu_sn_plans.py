@@ -2,7 +2,8 @@
 shapes where it can go wrong: one CTA for the only tree; one CTA per tree, and
 per 2 or 4 trees with the same factor; slots in shared or global memory; lower
 trees plus tasks above them, of one factor and of several; trees alone (a
-forest of small ones).  Against the host walk of the same fronts, and batches
+forest of small ones); test_cpu_sn_streams.py checks that the domains take these
+routes.  Against the host walk of the same fronts, and batches
 against single solves.
 
 Tolerance: the kernels' products are exact in FP64 and their sums differ from
@@ -16,6 +17,7 @@ import pytest
 
 from hierarchicaldd_b200 import domains
 from shim_ffi import load_shim
+from sn_routes import ROUTES, domain
 
 pytestmark = pytest.mark.gpu
 
@@ -26,33 +28,11 @@ def _fp(a):
     return a.ctypes.data_as(C.POINTER(C.c_float))
 
 
-def _domain(name):
-    if name == "one tree":              # interface systems of a few hundred unknowns: one CTA
-        return domains.small(16, 8, 3, seed=4), 2
-    if name == "pairs":                 # 2 trees per CTA
-        return domains.small((40, 36, 44), 8, 6, seed=4), 2
-    if name == "quads":                 # 4 trees per CTA
-        return domains.small((56, 56, 64), 8, 6, seed=4), 2
-    if name == "fronts in pairs":       # 2 trees per CTA; cut interface systems
-        return domains.small(96, 16, 20, seed=4), 3
-    if name == "slots in memory":       # 32^3 interiors: update slots do not fit
-        return domains.small(128, 32, 24, seed=4), 2
-    if name == "cut factors":           # few large trees: cut, members sharing coefficients
-        return domains.small(64, 32, 9, seed=4), 2
-    if name == "ragged":
-        return domains.small((33, 40, 41), 16, 5, seed=4), 2
-    # Many components: plans of thousands of tiny fronts, trees without fronts above.
-    d = domains.config5(16)
-    d.meta.update(vlevels=3, interior_smoothing=3, boundary_smoothing=3)
-    return domains.Domain(d.size, d.flags, d.rhs, (8, 8, 8), d.name, d.meta), 2
-
-
-@pytest.mark.parametrize("name", ["one tree", "pairs", "quads", "fronts in pairs", "slots in memory", "cut factors",
-                                  "ragged", "forest"])
+@pytest.mark.parametrize("name", ROUTES)
 def test_every_route_matches_the_host_walk_and_its_batches(name):
     from hierarchicaldd_b200 import _lib
     from hierarchicaldd_b200.solver import SPGrid_Domain_Decomposition_Solver
-    d, levels = _domain(name)
+    d, levels = domain(name)
     m = dict(d.meta)
     shim = load_shim()
     err = C.create_string_buffer(512)

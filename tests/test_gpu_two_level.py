@@ -9,7 +9,7 @@ against the oracle's two-level restatement:
   solution within 1e-5 relative L2 of the FP32 oracle's, on small and ragged
   domains;
 * the demo's own defaults (64^3 subdomains, so 32^3 V-cycle boxes on the
-  cluster kernel, vlevels 3, smoothing 1/3, sigma_levels 3) at 128^3 and at the
+  kernel, vlevels 3, smoothing 1/3, sigma_levels 3) at 128^3 and at the
   256^3 workload's domain, against the oracle's full solves in
   tests/golden/two_level_oracle.npz (tests/golden/make_two_level_fixture.py);
 * the solve server takes two-level domains (one system per context, whatever
