@@ -288,7 +288,10 @@ struct SolvePlan {
                PhaseHook* hook = nullptr) const;
     // With nrhs = 2 or 4 it solves that many systems at once: right-hand side
     // j at b_old + j ld_b, solution at x_old + j ld_x, one system's work beside
-    // the other's; each solution is bit-identical to its solve alone.
+    // the other's; each solution is bit-identical to its solve alone.  (Kernels
+    // that fed all systems from each coefficient they loaded were slower: whole
+    // solves of a batch of four took 70 ms at 64^3, 343 at 128^3 and 1176 at 192^3;
+    // these take 30, 122 and 431, and a solve alone 18, 58 and 151.)
     void solve(const PlanScratch& sc, const float* b_old, float* x_old, cudaStream_t s, long long& launches,
                PhaseHook* hook = nullptr, int nrhs = 1, long long ld_b = 0, long long ld_x = 0) const;
     // Scratch for another solve context (error word shared_err, or its own),

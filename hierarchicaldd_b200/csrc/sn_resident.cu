@@ -19,12 +19,16 @@
 //   on a loaded value.  With the same schedule but the records, gather lists
 //   and coefficients read where they are used, a tree level cost 5 to 7 us of
 //   dependent loads (102 us for the 64 16^3 interiors, n = 1423, of a 64^3
-//   domain); it now takes 40 us, against 92 us as separate forward and
-//   backward launches of one CTA per block of a front.  32^3 interiors: 170 us
-//   for the 64 of a 128^3 domain (345 before), 191 us for 216 (590 before).
-//   What is left is instruction issue: 16 conversions (4 cycles each on a
-//   scheduler) and 16 FP64 multiply-adds per 2 KB of coefficients and warp,
-//   about 560 cycles of set-up per product and 450 per barrier.
+//   domain); it now takes 38 us, against 92 us as separate forward and
+//   backward launches of one CTA per block of a front.  32^3 interiors: 169 us
+//   for the 64 of a 128^3 domain (345 before), 186 us for 216 (590 before).
+//   The price is memory: with headers, indices, rows and columns padded to the
+//   lanes and both directions stored, streams are three to four times the
+//   coefficients of both directions, 15 times for the tiny fronts of sparse domains.
+//   What is left is latency on four warps a scheduler: about 560 cycles of
+//   set-up per product and 450 per barrier.  The 32^3 interiors issue in 41 % of
+//   the cycles; the conversions of coefficients to FP64 (16 per 2 KB and warp)
+//   keep their pipe 40 % busy.
 // * Members of a class (trees whose factors are equal: most subdomains of a
 //   domain have the same interior matrix) share one stream, and up to K of
 //   them are solved by one CTA, which then feeds K products from every

@@ -19,17 +19,21 @@ constexpr int kPartMax = 4096;
 // coefficients do for its operations (the trees of sparse domains are thousands
 // of tiny fronts).  The cut grows with the plan so that its trees are about one
 // CTA per SM: larger ones would take longer than the task levels they save,
-// smaller ones leave more of those.  Measured (us per
-// solve at cuts of total/280 and at least 16000, total/250 and 36000,
-// total/170 and 48000): interface of 40x36x44, sub 8 (9 MB) 82, 81, 75; 64^3,
-// sub 16 (15 MB) 86, 87, 84; second level of 192^3, sub 32 (39 MB) 94, 90, 101;
-// 128^3 (63 MB) 121, 124, 119; sparse 128^3 43, 41, 31.
+// smaller ones leave more of those.  Measured (us per solve at cuts of total/280
+// and at least 16000, total/250 and 36000, total/220 and 48000 (these),
+// total/170 and 48000): level-0 interface of 40x36x44, sub 8: 78, 77, 73, 74;
+// 64^3, sub 16: 84, 82, 79, 79; 128^3, sub 32: 119, 120, 121, 117; 192^3: 272,
+// 271, 272, 273, its second level 160, 159, 164, 159 and third 89, 89, 90, 92;
+// second level of sparse 128^3 41, 36, 27, 28; two-level interiors 85, 84, 84, 88.
+// Which is best changes by a few per cent; the minimum matters most.
 constexpr double kCutMin = 48000, kCutMax = 200000, kCutShare = 220;
 // One CTA per whole tree takes as long as its largest tree's weight; cut, about
-// as long as kCutCost, and a kCutRate-th of all.  Measured (us
-// per solve): 8 interiors of 32^3 whole 158, cut 69; 16, 32 and 48 of them cut
-// 81, 104 and 153; 64 whole 165; a 16^3 domain's interface (564 unknowns) whole
-// 27, cut 43.
+// as long as kCutCost, and a kCutRate-th of all.  Measured (us per solve, whole
+// and cut): a 16^3 domain's interface (564 unknowns) 25 and 35; interiors of
+// 40x36x44 (sub 8) 21 and 24, of 64^3 (sub 16) 38 and 49, of 192^3 (216 of 32^3)
+// 186 and 356; bubble 48^3 second interface level 133 and 57, sparse 128^3 323 and
+// 28; 16 interiors of a two-level domain 158 and 63.  Near the line cutting can win
+// on the whole side too: the 64 interiors of 128^3 (sub 32) take 169 and 134.
 constexpr double kCutCost = 300000, kCutRate = 80;
 constexpr int kCutLen = 8192;
 

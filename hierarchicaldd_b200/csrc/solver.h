@@ -194,9 +194,9 @@ struct Solver {
 
     // Optional per-phase device timing with CUDA events on the solver stream
     // (categories: 0 V-cycle kernel, 1 Laplacian kernel, 2 PCG vector kernels,
-    // 3 interface gather/scatter, 4 sigma V-cycle (includes 6 and 7),
-    // 5 dense<->tile copies, 6 supernodal forward, 7 supernodal backward),
-    // with each phase's algorithmic bytes.
+    // 3 interface gather/scatter, 4 sigma V-cycle (includes 6),
+    // 5 dense<->tile copies, 6 supernodal solves, 7 none), with each phase's
+    // algorithmic bytes.
     static constexpr int kCats = 8;
     bool timing = false;
     double cat_ms[kCats] = {0};
