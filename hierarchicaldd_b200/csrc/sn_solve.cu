@@ -49,6 +49,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
+#include <exception>
 #include <map>
 #include <numeric>
 #include <string>
@@ -473,17 +474,17 @@ void SolvePlan::build(const std::vector<const SnFactor*>& factors, const std::ve
         std::vector<std::pair<const SnFactor* const, FactorCut>*> each;
         for (auto& c : cuts) each.push_back(&c);
         const double cap = cut_weight(total) / shrink;
-        std::string failed;
+        std::exception_ptr failed;
 #pragma omp parallel for schedule(dynamic)
         for (size_t i = 0; i < each.size(); ++i) {
             try {
                 each[i]->second = cut_trees(*each[i]->first, cap);
-            } catch (const std::exception& e) {
+            } catch (...) {
 #pragma omp critical
-                failed = e.what();
+                failed = std::current_exception();
             }
         }
-        if (!failed.empty()) throw Error(HDD_ERR_UNSUPPORTED, failed);
+        if (failed) std::rethrow_exception(failed);
     }
     std::vector<ResidentPlan::Shape> shapes;
     std::vector<std::vector<ResidentPlan::Member>> members;
